@@ -114,6 +114,21 @@ __device__ __forceinline__ int64_t bisect_left(const uint64_t* __restrict__ a, i
   return lo;
 }
 
+// 1/x for a positive, finite, normal x well inside the range (2^-1000 < x < 2^1000; other values
+// take the plain division). The FP64 pipe issues 1.6 lanes a clock and SM, so kernels of many
+// reciprocals are bound by it; the plain division is about ten of its operations, this is
+// three: the PTX approximation (rcp.approx.ftz.f64, a relative error e of about 2^-20) and one
+// third-order step y (1 + e + e^2) of the Neumann series of 1/(1 - e) (Householder's method for
+// 1/x), whose truncation e^3 is below the rounding of the result.
+__device__ __forceinline__ double rcp_f64(double x) {
+  const unsigned ex = ((unsigned)__double2hiint(x) >> 20);  // sign and exponent
+  if (ex - 23u > 2000u) return 1.0 / x;                     // outside [2^-1000, 2^1000), zero, negative, NaN
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
 // ---- deterministic block reduction -------------------------------------------------------
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double* smem /*[NT/32]*/) {

@@ -4,6 +4,7 @@
 // function from Krylov spectral weights (gf_greater / gf_lesser, cmpy/exactdiag.py:248-302)
 // and its Laplace transform to complex frequencies (fourier_t2z, cmpy/exactdiag.py:311-316).
 // Complex numbers are interleaved (re, im) FP64 pairs.
+#include <algorithm>
 #include <cmath>
 
 #include "ed_plan.cuh"
@@ -46,38 +47,60 @@ __global__ void k_lehmann_poles(const double* __restrict__ e, int64_t nd, const 
   }
 }
 
-// g[z] += sum_k coef_k / (z - pole_k); one block per frequency chunk, terms staged in smem
-constexpr int LEH_T = 1024;
-__global__ void k_lehmann_sum(const double* __restrict__ coef, const double* __restrict__ pole, int64_t nt,
-                              const double2* __restrict__ z, int64_t nz, double2* __restrict__ g) {
-  __shared__ double sc[LEH_T], sp[LEH_T];
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// part[q][z] = sum of coef_k / (z - pole_k) over the terms of chunk q (blockIdx.y), one thread
+// per frequency, the terms staged in shared memory. Bound by the FP64 pipe (eight operations a
+// term and frequency): the terms are split over as many blocks as fill the GPU, because the
+// frequencies alone do not: 512 of them are four blocks, which took 8.4 ms for the mean sector
+// pair of the 6-site chain. Split, its thermal G over all sectors went from 567 to 222 ms.
+constexpr int LEH_NT = 128;  // frequencies per block
+constexpr int LEH_T = 256;   // terms per tile
+__global__ void __launch_bounds__(LEH_NT) k_lehmann_sum(const double* __restrict__ coef, const double* __restrict__ pole,
+                                                        int64_t nt, int64_t chunk, const double2* __restrict__ z,
+                                                        int64_t nz, double2* __restrict__ part) {
+  __shared__ double2 st[LEH_T];
+  const int64_t i = blockIdx.x * (int64_t)LEH_NT + threadIdx.x;
   const double2 zi = i < nz ? z[i] : make_double2(0.0, 1.0);
   const double zm2 = zi.y * zi.y;
-  double gr = 0.0, gm = 0.0;
-  for (int64_t t0 = 0; t0 < nt; t0 += LEH_T) {
+  const int64_t k0 = blockIdx.y * chunk, k1 = min(nt, k0 + chunk);
+  double gr = 0.0, gs = 0.0;
+  for (int64_t t0 = k0; t0 < k1; t0 += LEH_T) {
+    const int tn = (int)min((int64_t)LEH_T, k1 - t0);
     __syncthreads();
-    for (int t = threadIdx.x; t < LEH_T; t += blockDim.x) {
-      const int64_t k = t0 + t;
-      sc[t] = k < nt ? coef[k] : 0.0;
-      sp[t] = k < nt ? pole[k] : 0.0;
-    }
+    for (int t = threadIdx.x; t < tn; t += LEH_NT) st[t] = make_double2(coef[t0 + t], pole[t0 + t]);
     __syncthreads();
-    const int tn = (int)((nt - t0) < LEH_T ? (nt - t0) : LEH_T);
+#pragma unroll 4
     for (int t = 0; t < tn; ++t) {
-      const double c = sc[t];
-      if (c == 0.0) continue;
-      const double ar = zi.x - sp[t];
-      const double inv = c / (ar * ar + zm2);
+      const double2 cp = st[t];
+      if (cp.x == 0.0) continue;  // uniform over the block
+      const double ar = zi.x - cp.y;
+      const double inv = cp.x * rcp_f64(fma(ar, ar, zm2));
       gr = fma(ar, inv, gr);
-      gm = fma(-zi.y, inv, gm);
+      gs += inv;
     }
   }
-  if (i < nz) {
-    double2 r = g[i];
-    r.x += gr;
-    r.y += gm;
-    g[i] = r;
+  if (i < nz) part[blockIdx.y * nz + i] = make_double2(gr, -zi.y * gs);
+}
+
+// g[z] += the chunk sums, one warp per frequency, in a fixed order
+__global__ void __launch_bounds__(LEH_NT) k_lehmann_reduce(const double2* __restrict__ part, int nq, int64_t nz,
+                                                           double2* __restrict__ g) {
+  const int64_t i = (blockIdx.x * (int64_t)LEH_NT + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (i >= nz) return;
+  double r = 0.0, m = 0.0;
+  for (int q = lane; q < nq; q += 32) {
+    const double2 v = part[q * nz + i];
+    r += v.x;
+    m += v.y;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    r += __shfl_xor_sync(0xffffffffu, r, o);
+    m += __shfl_xor_sync(0xffffffffu, m, o);
+  }
+  if (lane == 0) {
+    g[i].x += r;
+    g[i].y += m;
   }
 }
 
@@ -214,14 +237,21 @@ ED_API ed_status ed_lehmann_accumulate(const double* d_e, int64_t nd, const doub
   ED_TRY(device_context(&ctx));
   cudaStream_t s = as_stream(stream);
   const int64_t nt = nd * ndp;
+  // chunks of terms: eight blocks per SM over all frequencies, at least one tile of terms each
+  const int64_t zb = (nz + LEH_NT - 1) / LEH_NT;
+  int64_t nq = std::min<int64_t>((nt + LEH_T - 1) / LEH_T, std::max<int64_t>(1, (int64_t)ctx->num_sms * 8 / zb));
+  const int64_t chunk = ((nt + nq - 1) / nq + LEH_T - 1) / LEH_T * LEH_T;
+  nq = (nt + chunk - 1) / chunk;
   double *coef = nullptr, *pole = nullptr;
-  ED_CUDA(cudaMallocAsync(&coef, nt * sizeof(double), s));
-  ED_CUDA(cudaMallocAsync(&pole, nt * sizeof(double), s));
+  double2* part = nullptr;
+  ED_CUDA(cudaMallocAsync(&coef, (2 * nt + 2 * nq * nz) * sizeof(double), s));
+  pole = coef + nt;
+  part = (double2*)(coef + 2 * nt);
   k_lehmann_poles<<<grid_for(nt, 256, ctx->num_sms * 8), 256, 0, s>>>(d_e, nd, d_ep, ndp, d_ov, beta, emin, coef, pole);
-  k_lehmann_sum<<<(unsigned)((nz + 127) / 128), 128, 0, s>>>(coef, pole, nt, (const double2*)d_z, nz, (double2*)d_g);
-  ED_CHECK_LAUNCH_N("ed_lehmann_accumulate", 2);
+  k_lehmann_sum<<<dim3((unsigned)zb, (unsigned)nq), LEH_NT, 0, s>>>(coef, pole, nt, chunk, (const double2*)d_z, nz, part);
+  k_lehmann_reduce<<<(unsigned)((nz * 32 + LEH_NT - 1) / LEH_NT), LEH_NT, 0, s>>>(part, (int)nq, nz, (double2*)d_g);
+  ED_CHECK_LAUNCH_N("ed_lehmann_accumulate", 3);
   ED_CUDA(cudaFreeAsync(coef, s));
-  ED_CUDA(cudaFreeAsync(pole, s));
   return ED_OK;
 }
 
