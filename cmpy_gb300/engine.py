@@ -635,6 +635,28 @@ def tevo_sum(lam, w, e0: float, sign: int, times, out: torch.Tensor | None = Non
     return g
 
 
+def tevo_krylov(alpha, beta, norm2: float, e0: float, sign: int, times) -> torch.Tensor:
+    """-i*sign * norm2 * <e1|exp(-i sign (T - e0) t)|e1> of the Lanczos tridiagonal T = (alpha[0..m),
+    beta[1..m)) for every t (complex128 on device): by a Chebyshev expansion, or from the
+    eigenpairs of T where the expansion would be too long."""
+    a = _as_dev_f64(alpha).reshape(-1)
+    b = _as_dev_f64(beta).reshape(-1)
+    m = a.numel()
+    if b.numel() < m:
+        raise ValueError("beta needs m entries (beta[0] unused)")
+    th = times.detach().cpu().numpy() if isinstance(times, torch.Tensor) else np.asarray(times, dtype=np.float64)
+    tt = _as_dev_f64(times).reshape(-1)
+    g = torch.empty(tt.numel(), dtype=torch.complex128, device=device())
+    done = C.c_int()
+    t_max = float(np.max(np.abs(th))) if th.size else 0.0
+    N.check(N.lib().ed_tevo_krylov(N.ptr(a), N.ptr(b), m, float(norm2), float(e0), int(sign), N.ptr(tt), tt.numel(),
+                                   t_max, N.ptr(torch.view_as_real(g)), 0, C.byref(done), _stream()))
+    if done.value:
+        return g
+    lam, U = tridiag_eigh(a, b[:m])
+    return tevo_sum(lam, norm2 * U[0, :] ** 2, e0, sign, tt, out=None)
+
+
 def laplace_t2z(times, gf_t, z, method: str = "lin") -> torch.Tensor:
     """int_{t_0}^{t_last} e^{izt} g(t) dt of samples g(t_j) (piecewise-linear "lin" or "trapz")."""
     tt = _as_dev_f64(times).reshape(-1)

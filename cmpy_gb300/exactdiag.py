@@ -371,7 +371,7 @@ def _tevo_part(model, gs, times: np.ndarray, pos: int, sigma: int, delta: int, n
     """-i e^{iE0 t}<gs|c e^{-iHt} c^dag|gs> (delta=+1) or +i e^{-iE0 t}<gs|c^dag e^{iHt} c|gs>
     (delta=-1) on the device. The reference propagates with scipy expm_multiply; here the
     Lanczos tridiagonal T_m of the start vector gives <phi|e^{-iHt}|phi> = |phi|^2 e1^T
-    e^{-iT_m t} e1, i.e. a sum over the eigenpairs of T_m (exact once m reaches the dimension,
+    e^{-iT_m t} e1, evaluated by a Chebyshev expansion in T_m (exact once m reaches the dimension,
     and converged long before that for ||H|| t << m)."""
     nb = _neighbour(model, gs.n_up, gs.n_dn, sigma, delta)
     if nb is None:
@@ -383,12 +383,9 @@ def _tevo_part(model, gs, times: np.ndarray, pos: int, sigma: int, delta: int, n
     steps = tplan.dim if n_lev is None else min(int(n_lev), tplan.dim)
     a, b, nrm = E.lanczos_coeffs(tplan, phi, max_steps=steps)
     m = a.numel()
-    tt = E._as_dev_f64(times)
     if m == 0 or nrm == 0.0:
-        return torch.zeros(tt.numel(), dtype=torch.complex128, device=E.device())
-    lam, U = E.tridiag_eigh(a[:m], b[:m])
-    w = (nrm * nrm) * U[0, :] ** 2
-    return E.tevo_sum(lam, w, float(gs.energy), 1 if delta > 0 else -1, tt)
+        return torch.zeros(len(times), dtype=torch.complex128, device=E.device())
+    return E.tevo_krylov(a, b, nrm * nrm, float(gs.energy), 1 if delta > 0 else -1, times)
 
 
 def _tevo(model, gs, start, stop, num, pos, sigma, delta, n_lev, jw_sign):

@@ -553,6 +553,16 @@ ED_API ed_status ed_tevo_sum(const double* d_lam, const double* d_w, int64_t m, 
                              const double* d_t, int64_t n_t, double* d_out, int accumulate,
                              ed_stream_t stream);
 
+/* The same function from the Lanczos coefficients themselves, T = (alpha[0..m), beta[1..m)) and
+ * norm2 the squared norm of the start vector: the Chebyshev expansion of exp(-i sign (T - e0) t)
+ * instead of the eigenpairs of T. t_abs_max bounds |t_n| (host value). *h_done = 0 (nothing
+ * written) when the expansion does not suit the input: m > 4096, or an order (|t| times half the
+ * spectral width, and some) above 16384 or above both 7 m and 400; the caller then takes ed_tridiag_eigh and
+ * ed_tevo_sum. Synchronises the stream once. */
+ED_API ed_status ed_tevo_krylov(const double* d_alpha, const double* d_beta, int m, double norm2, double e0, int sign,
+                                const double* d_t, int64_t n_t, double t_abs_max, double* d_out, int accumulate,
+                                int* h_done, ed_stream_t stream);
+
 /* Laplace transform G(z) = int_{t_0}^{t_last} e^{i z t} g(t) dt of complex samples g(t_j) to n_z
  * complex frequencies — fourier_t2z (cmpy/exactdiag.py:311-316), which calls
  * gftool.fourier.tt2z. method 0: exact integral of the piecewise-linear interpolant of g
