@@ -160,7 +160,7 @@ def groundstate_all_sectors(model, max_steps: int = 300, tol: float = 1e-12, che
     batched counterpart of cmpy's compute_groundstate, exactdiag.py:24-43).
     Returns (fillings, BatchResult)."""
     fillings = list(model.basis.iter_fillings())
-    plans = [model.plan(nu, nd) for nu, nd in fillings]
+    plans = model.plans(fillings)
     b = Batch(plans)
     if tune:
         b.tune(min(40, max_steps))

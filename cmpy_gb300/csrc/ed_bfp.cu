@@ -1263,85 +1263,65 @@ static void free_stripe(StripeTables& T) {
 // order of stripe_order, and per renumbered column its + then - partners as byte offsets 16*j
 // of the interleaved row pair, two per word; every column of a 64-column chunk has the chunk's
 // largest + and - pair counts (padded with the zero slot 16*nd). CMPY_ED_DNC=0 disables it.
-static ed_status build_dncompact(ed_plan_s* p, BfpTables& B, const std::vector<int32_t>& doff,
-                                 const std::vector<int32_t>& didx, const std::vector<double>& dcoef,
-                                 const std::vector<int32_t>& edi, const std::vector<int64_t>& edf, cudaStream_t s) {
+static void build_dncompact(ed_plan_s* p, BfpTables& B, const HostTable& h, const std::vector<int32_t>& edi,
+                            const std::vector<int64_t>& edf, DeviceArena& arena) {
   DnCompactTables& T = B.dc;
   T = DnCompactTables();
   const char* env = getenv("CMPY_ED_DNC");
-  if (env && atoi(env) == 0) return ED_OK;
+  if (env && atoi(env) == 0) return;
   const int64_t nu = p->num_up, nd = p->num_dn;
-  if (nd < 2 || nd % 2 || nd >= 4096) return ED_OK;  // the single-pass kernel's limits
+  if (nd < 2 || nd % 2 || nd >= 4096) return;  // the single-pass kernel's limits
   StripeSide sd;
-  if (!stripe_order(nd, doff, didx, dcoef, &sd)) return ED_OK;
+  if (!stripe_order(nd, h.off, h.idx, h.coef, &sd, false)) return;
   std::vector<int32_t> inv(nd);
   for (int64_t i = 0; i < nd; ++i) inv[sd.perm[i]] = (int32_t)i;
   const int64_t nchunk = (nd + 63) / 64;
-  std::vector<std::vector<uint32_t>> pos(nd), neg(nd);
-  for (int64_t i = 0; i < nd; ++i) {
-    const int64_t v = sd.perm[i];
-    for (int32_t k = doff[v]; k < doff[v + 1]; ++k) {
-      if (dcoef[k] == 0.0) continue;
-      (dcoef[k] > 0.0 ? pos[i] : neg[i]).push_back(16u * (uint32_t)inv[didx[k]]);
-    }
-  }
   std::vector<uint16_t> chunk(nchunk);
   int rows = 0;
   for (int64_t c = 0; c < nchunk; ++c) {
     int pp = 0, pn = 0;
     for (int64_t i = c * 64; i < std::min<int64_t>(nd, (c + 1) * 64); ++i) {
-      pp = std::max(pp, (int)(pos[i].size() + 1) / 2);
-      pn = std::max(pn, (int)(neg[i].size() + 1) / 2);
+      pp = std::max(pp, (int)(sd.meta[i] & 0xff));
+      pn = std::max(pn, (int)(sd.meta[i] >> 8));
     }
     chunk[c] = (uint16_t)(pp | (pn << 8));
     rows = std::max(rows, pp + pn);
   }
   rows = std::max(rows, 1);
-  if (mv3_layout(nd, rows, B.max_up).total + MV3_STATIC_SMEM > (size_t)p->ctx->smem_optin) return ED_OK;
+  if (mv3_layout(nd, rows, B.max_up).total + MV3_STATIC_SMEM > (size_t)p->ctx->smem_optin) return;
   const uint32_t zero = 16u * (uint32_t)nd;
   std::vector<uint32_t> tab((size_t)rows * nd, zero | (zero << 16));
+  std::vector<uint64_t> sdn(nd);
   for (int64_t i = 0; i < nd; ++i) {
-    const int pp = chunk[i / 64] & 0xff;
-    auto put = [&](const std::vector<uint32_t>& lst, int row0) {
-      for (size_t e = 0; e < lst.size(); e += 2) {
-        const uint32_t lo = lst[e], hi = e + 1 < lst.size() ? lst[e + 1] : zero;
-        tab[(size_t)(row0 + e / 2) * nd + i] = lo | (hi << 16);
-      }
-    };
-    put(pos[i], 0);
-    put(neg[i], pp);
+    const int64_t v = sd.perm[i];
+    sdn[i] = h.states[v];
+    int np = 0, nn = 0;
+    for (int32_t k = h.off[v]; k < h.off[v + 1]; ++k) {
+      if (h.coef[k] == 0.0) continue;
+      const int e = h.coef[k] > 0.0 ? np++ : 2 * (chunk[i / 64] & 0xff) + nn++;  // entry e: half e & 1 of row e / 2
+      uint32_t& w = tab[(size_t)(e / 2) * nd + i];
+      const uint32_t o = 16u * (uint32_t)inv[h.idx[k]];
+      w = (e & 1) ? (w & 0xffffu) | (o << 16) : (w & 0xffff0000u) | o;
+    }
   }
   std::vector<int32_t> ident(nu);
   for (int64_t i = 0; i < nu; ++i) ident[i] = (int32_t)i;
-  std::vector<uint64_t> st_dn(nd), sdn(nd);
-  ED_CUDA(cudaMemcpyAsync(st_dn.data(), p->dn.states, nd * 8, cudaMemcpyDeviceToHost, s));
-  ED_CUDA(cudaStreamSynchronize(s));
-  for (int64_t i = 0; i < nd; ++i) sdn[i] = st_dn[sd.perm[i]];
-  ED_TRY(dev_upload((void**)&T.tab, tab.data(), tab.size() * 4, s));
-  ED_TRY(dev_upload((void**)&T.chunk, chunk.data(), chunk.size() * 2, s));
-  ED_TRY(dev_upload((void**)&T.perm_up, ident.data(), ident.size() * 4, s));
-  ED_TRY(dev_upload((void**)&T.perm_dn, sd.perm.data(), sd.perm.size() * 4, s));
-  ED_TRY(dev_upload((void**)&T.s_dn, sdn.data(), sdn.size() * 8, s));
+  arena.add(&T.tab, tab.data(), tab.size() * 4);
+  arena.add(&T.chunk, chunk.data(), chunk.size() * 2);
+  arena.add(&T.perm_up, ident.data(), ident.size() * 4);
+  arena.add(&T.perm_dn, sd.perm.data(), sd.perm.size() * 4);
+  arena.add(&T.s_dn, sdn.data(), sdn.size() * 8);
   if (!B.diag64) {
     std::vector<int32_t> b(nd);
     for (int64_t i = 0; i < nd; ++i) b[i] = edi[sd.perm[i]];
-    ED_TRY(dev_upload((void**)&T.e_dn, b.data(), b.size() * 4, s));
-    ED_CUDA(cudaStreamSynchronize(s));
+    arena.add(&T.e_dn, b.data(), b.size() * 4);
   } else {
     std::vector<int64_t> b(nd);
     for (int64_t i = 0; i < nd; ++i) b[i] = edf[sd.perm[i]];
-    ED_TRY(dev_upload((void**)&T.f_dn, b.data(), b.size() * 8, s));
-    ED_CUDA(cudaStreamSynchronize(s));
+    arena.add(&T.f_dn, b.data(), b.size() * 8);
   }
   T.rows = rows;
   T.on = 1;
-  return ED_OK;
-}
-
-static void free_dncompact(DnCompactTables& T) {
-  cudaFree(T.tab); cudaFree(T.chunk); cudaFree(T.perm_up); cudaFree(T.perm_dn);
-  cudaFree(T.s_dn); cudaFree(T.e_dn); cudaFree(T.f_dn);
-  T = DnCompactTables();
 }
 
 // Tables of the banded two-pass matvec (ed_sweep.cuh); leaves B.sw.on = 0 when the sector does
@@ -1413,24 +1393,51 @@ static void free_sweep(SweepTables& W) {
   W = SweepTables();
 }
 
-ed_status build_bfp(ed_plan_s* p, cudaStream_t s) {
-  BfpTables& B = p->bfp;
-  B = BfpTables();
-  if (p->kind != 0 || p->dim == 0) return ED_OK;
-  // one hopping magnitude
-  double tmag = 0.0;
+// per-state energies in the plan's diagonal mode: integers * 2^-F, or fixed point with Fd bits
+static void bfp_energies(const BfpTables& B, const std::vector<double>& eu, const std::vector<double>& edn,
+                         std::vector<int32_t>& eui, std::vector<int32_t>& edi, std::vector<int64_t>& euf,
+                         std::vector<int64_t>& edf) {
+  auto as_int = [&](const std::vector<double>& e, std::vector<int32_t>& o) {
+    o.resize(e.size());
+    for (size_t i = 0; i < e.size(); ++i) o[i] = (int32_t)std::ldexp(e[i], B.F);
+  };
+  auto as_fx = [&](const std::vector<double>& e, std::vector<int64_t>& o) {
+    o.resize(e.size());
+    for (size_t i = 0; i < e.size(); ++i) o[i] = std::llrint(std::ldexp(e[i], B.Fd));
+  };
+  if (!B.diag64) {
+    as_int(eu, eui);
+    as_int(edn, edi);
+  } else {
+    as_fx(eu, euf);
+    as_fx(edn, edf);
+  }
+}
+
+// one hopping magnitude, and rows that fit the matvec's 16-bit shared-memory slots
+static bool one_hop(const ed_plan_s* p, double* tmag) {
+  *tmag = 0.0;
   for (double h : p->hop) {
     if (h == 0.0) continue;
-    if (tmag == 0.0) tmag = std::fabs(h);
-    else if (std::fabs(h) != tmag) return ED_OK;
+    if (*tmag == 0.0) *tmag = std::fabs(h);
+    else if (std::fabs(h) != *tmag) return false;
   }
-  if (p->num_dn * 2 + 1 > 65535) return ED_OK;  // 16-bit shared-memory slots
-  if ((2 * p->num_dn + 1) * 8 > 200 * 1024) return ED_OK;
+  return true;
+}
+
+bool bfp_possible(const ed_plan_s* p) {
+  double tmag;
+  return p->kind == 0 && p->dim > 0 && one_hop(p, &tmag) && p->num_dn * 2 + 1 <= 65535 &&
+         (2 * p->num_dn + 1) * 8 <= 200 * 1024;
+}
+
+ed_status build_bfp(ed_plan_s* p, const HostTable& hu, const HostTable& hd, DeviceArena& arena) {
+  BfpTables& B = p->bfp;
+  B = BfpTables();
+  double tmag;
+  if (!bfp_possible(p) || !one_hop(p, &tmag)) return ED_OK;
   // coefficients: per-state energies (exact FP64 sums), U and t as integers * 2^-F
-  std::vector<double> eu(p->num_up), edn(p->num_dn);
-  ED_CUDA(cudaMemcpyAsync(eu.data(), p->up.energy, p->num_up * sizeof(double), cudaMemcpyDeviceToHost, s));
-  ED_CUDA(cudaMemcpyAsync(edn.data(), p->dn.energy, p->num_dn * sizeof(double), cudaMemcpyDeviceToHost, s));
-  ED_CUDA(cudaStreamSynchronize(s));
+  const std::vector<double>&eu = hu.energy, &edn = hd.energy;
   // mode 0: t, U and the state energies are integers * 2^-F (exact diagonal)
   int F = -1;
   for (int f = 0; f <= 40 && F < 0; ++f) {
@@ -1448,22 +1455,10 @@ ed_status build_bfp(ed_plan_s* p, cudaStream_t s) {
     if (F < 0) return ED_OK;
     diag64 = 1;
   }
-  // row tables (host copies of the FP64 tables)
-  std::vector<int32_t> uoff(p->num_up + 1), uidx(p->up.nnz), doff(p->num_dn + 1), didx(p->dn.nnz);
-  std::vector<double> ucoef(p->up.nnz), dcoef(p->dn.nnz);
-  std::vector<int16_t> dbond(p->dn.nnz);
-  ED_CUDA(cudaMemcpyAsync(uoff.data(), p->up.off, uoff.size() * 4, cudaMemcpyDeviceToHost, s));
-  ED_CUDA(cudaMemcpyAsync(doff.data(), p->dn.off, doff.size() * 4, cudaMemcpyDeviceToHost, s));
-  if (p->up.nnz) {
-    ED_CUDA(cudaMemcpyAsync(uidx.data(), p->up.idx, uidx.size() * 4, cudaMemcpyDeviceToHost, s));
-    ED_CUDA(cudaMemcpyAsync(ucoef.data(), p->up.coef, ucoef.size() * 8, cudaMemcpyDeviceToHost, s));
-  }
-  if (p->dn.nnz) {
-    ED_CUDA(cudaMemcpyAsync(didx.data(), p->dn.idx, didx.size() * 4, cudaMemcpyDeviceToHost, s));
-    ED_CUDA(cudaMemcpyAsync(dcoef.data(), p->dn.coef, dcoef.size() * 8, cudaMemcpyDeviceToHost, s));
-    ED_CUDA(cudaMemcpyAsync(dbond.data(), p->dn.bond, dbond.size() * 2, cudaMemcpyDeviceToHost, s));
-  }
-  ED_CUDA(cudaStreamSynchronize(s));
+  // row tables (the FP64 tables)
+  const std::vector<int32_t>&uoff = hu.off, &uidx = hu.idx, &doff = hd.off, &didx = hd.idx;
+  const std::vector<double>&ucoef = hu.coef, &dcoef = hd.coef;
+  const std::vector<int16_t>& dbond = hd.bond;
   const int64_t nu = p->num_up, nd = p->num_dn;
   std::vector<int32_t> boff(nu + 1), bnpos(nu), bidx;
   bidx.reserve(p->up.nnz);
@@ -1549,13 +1544,9 @@ ed_status build_bfp(ed_plan_s* p, cudaStream_t s) {
   while (std::ldexp(1.0, lb) <= bound) ++lb;  // bound < 2^lb
   const int m_in = std::min(56, 62 - lb);
   if (m_in < 48) return ED_OK;
-  std::vector<int32_t> eui, edi;
-  std::vector<int64_t> euf, edf;
+  B.diag64 = diag64;
+  B.F = F;
   if (!diag64) {
-    eui.resize(nu);
-    edi.resize(nd);
-    for (int64_t i = 0; i < nu; ++i) eui[i] = (int32_t)std::ldexp(eu[i], F);
-    for (int64_t i = 0; i < nd; ++i) edi[i] = (int32_t)std::ldexp(edn[i], F);
     for (int i = 0; i < p->n_sites; ++i) B.u_int[i] = (int32_t)std::ldexp(p->u[i], F);
     B.u0_int = p->n_sites ? B.u_int[0] : 0;
   } else {
@@ -1564,28 +1555,21 @@ ed_status build_bfp(ed_plan_s* p, cudaStream_t s) {
     while (std::ldexp(1.0, ld) <= diag_max) ++ld;
     B.Fd = 61 - ld;
     if (B.Fd - F < 1 || B.Fd - F > 63) return ED_OK;
-    euf.resize(nu);
-    edf.resize(nd);
-    for (int64_t i = 0; i < nu; ++i) euf[i] = std::llrint(std::ldexp(eu[i], B.Fd));
-    for (int64_t i = 0; i < nd; ++i) edf[i] = std::llrint(std::ldexp(edn[i], B.Fd));
     for (int i = 0; i < p->n_sites; ++i) B.u_fx[i] = std::llrint(std::ldexp(p->u[i], B.Fd));
     B.u0_fx = p->n_sites ? B.u_fx[0] : 0;
   }
-  B.diag64 = diag64;
-  B.F = F;
+  std::vector<int32_t> eui, edi;
+  std::vector<int64_t> euf, edf;
+  bfp_energies(B, eu, edn, eui, edi, euf, edf);
   B.m_in = m_in;
   B.max_dn = max_dn;
   B.vec2 = (nd % 2 == 0) ? 1 : 0;
-  auto up = [&](auto** dst, const void* src, size_t bytes) -> ed_status {
-    ED_CUDA(cudaMalloc((void**)dst, std::max<size_t>(bytes, 8)));
-    if (bytes) ED_CUDA(cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, s));
-    return ED_OK;
-  };
-  ED_TRY(up(&B.up_off, boff.data(), boff.size() * 4));
-  ED_TRY(up(&B.up_npos, bnpos.data(), bnpos.size() * 4));
-  ED_TRY(up(&B.up_idx, bidx.data(), bidx.size() * 4));
-  ED_TRY(up(&B.dn_tab, tab.data(), tab.size() * 2));
-  ED_TRY(up(&B.dn_btab2, btab2.data(), btab2.size() * 4));
+  auto up = [&](auto** dst, const void* src, size_t bytes) { arena.add(dst, src, bytes); };
+  up(&B.up_off, boff.data(), boff.size() * 4);
+  up(&B.up_npos, bnpos.data(), bnpos.size() * 4);
+  up(&B.up_idx, bidx.data(), bidx.size() * 4);
+  up(&B.dn_tab, tab.data(), tab.size() * 2);
+  up(&B.dn_btab2, btab2.data(), btab2.size() * 4);
   B.n_b2 = n_rows / 2;
   B.n_b2pos = pos_pad / 2;
   B.max_up = max_up;
@@ -1606,34 +1590,51 @@ ed_status build_bfp(ed_plan_s* p, cudaStream_t s) {
       cnt[(size_t)r * 4 + 1] = cn;
       cnt[(size_t)r * 4 + 2] = (cn - (n - np)) - (cp - np);  // padding copies of the row, with sign
     }
-    ED_TRY(up(&B.up_lst, lst.data(), lst.size() * 4));
-    ED_TRY(up(&B.up_cnt, cnt.data(), cnt.size() * 4));
+    up(&B.up_lst, lst.data(), lst.size() * 4);
+    up(&B.up_cnt, cnt.data(), cnt.size() * 4);
     B.up_lstride = ls;
   }
   if (!diag64) {
-    ED_TRY(up(&B.e_up_int, eui.data(), eui.size() * 4));
-    ED_TRY(up(&B.e_dn_int, edi.data(), edi.size() * 4));
+    up(&B.e_up_int, eui.data(), eui.size() * 4);
+    up(&B.e_dn_int, edi.data(), edi.size() * 4);
   } else {
-    ED_TRY(up(&B.e_up_fx, euf.data(), euf.size() * 8));
-    ED_TRY(up(&B.e_dn_fx, edf.data(), edf.size() * 8));
+    up(&B.e_up_fx, euf.data(), euf.size() * 8);
+    up(&B.e_dn_fx, edf.data(), edf.size() * 8);
   }
-  ED_CUDA(cudaStreamSynchronize(s));
-  ED_TRY(build_sweep(p, B, uoff, uidx, ucoef, doff, didx, dcoef, eui, edi, euf, edf, s));
-  ED_TRY(build_stripe(p, B, uoff, uidx, ucoef, doff, didx, dcoef, eui, edi, euf, edf, s));
-  ED_TRY(build_dncompact(p, B, doff, didx, dcoef, edi, edf, s));
+  build_dncompact(p, B, hd, edi, edf, arena);
   B.eligible = 1;
   return ED_OK;
 }
 
-void free_bfp(ed_plan_s* p) {
+// The tables of the two-pass variants: built when one of them is asked for (5, 6) or when the
+// single-pass kernels do not fit (5), from the plan's device tables; synchronous.
+ed_status build_two_pass(ed_plan_s* p, bool sweep, bool stripe, cudaStream_t s) {
   BfpTables& B = p->bfp;
-  cudaFree(B.up_off); cudaFree(B.up_npos); cudaFree(B.up_idx); cudaFree(B.dn_tab); cudaFree(B.dn_btab2);
-  cudaFree(B.up_lst); cudaFree(B.up_cnt);
-  cudaFree(B.e_up_int); cudaFree(B.e_dn_int); cudaFree(B.e_up_fx); cudaFree(B.e_dn_fx);
-  free_sweep(B.sw);
-  free_stripe(B.sp);
-  free_dncompact(B.dc);
-  B = BfpTables();
+  sweep = sweep && B.eligible && !B.sw_tried;
+  stripe = stripe && B.eligible && !B.sp_tried;
+  if (!sweep && !stripe) return ED_OK;
+  HostTable hu, hd;
+  ED_TRY(download_table(p->up, &hu, s));
+  ED_TRY(download_table(p->dn, &hd, s));
+  std::vector<int32_t> eui, edi;
+  std::vector<int64_t> euf, edf;
+  bfp_energies(B, hu.energy, hd.energy, eui, edi, euf, edf);
+  if (sweep) {
+    ED_TRY(build_sweep(p, B, hu.off, hu.idx, hu.coef, hd.off, hd.idx, hd.coef, eui, edi, euf, edf, s));
+    B.sw_tried = true;
+  }
+  if (stripe) {
+    ED_TRY(build_stripe(p, B, hu.off, hu.idx, hu.coef, hd.off, hd.idx, hd.coef, eui, edi, euf, edf, s));
+    B.sp_tried = true;
+  }
+  return ED_OK;
+}
+
+void free_bfp(ed_plan_s* p) {
+  // the single-pass tables live in the plan's arena
+  free_sweep(p->bfp.sw);
+  free_stripe(p->bfp.sp);
+  p->bfp = BfpTables();
 }
 
 // first-wait limit of the bulk-copy matvecs (polls); 0 selects MV3_WAIT_LIMIT
@@ -1722,6 +1723,15 @@ static int matvec_variant(const ed_plan_s* p) {
   if (v3_ok) return 3;
   if (v5_ok) return 5;
   return v2_ok ? 2 : 1;
+}
+
+// at plan creation: the sweep's tables when the single-pass kernels do not fit, either variant's
+// when the environment asks for it
+ed_status build_default_two_pass(ed_plan_s* p, cudaStream_t s) {
+  if (!p->bfp.eligible) return ED_OK;
+  const char* e = getenv("CMPY_ED_MATVEC");
+  const int forced = e ? atoi(e) : 0;
+  return build_two_pass(p, forced == 5 || matvec_variant(p) < 3, forced == 6, s);
 }
 
 // CTAs of the stripe passes (persistent, as many as the SMs hold)
@@ -2384,6 +2394,7 @@ ED_API int ed_plan_matvec_variant(ed_plan p) { return (p && p->bfp.eligible) ? m
 ED_API ed_status ed_plan_set_matvec_variant(ed_plan p, int variant) {
   ED_TRY(check_plan(p));
   if (variant < 0 || variant > 7) return fail(ED_ERR_INVALID_ARG, "variant must be in [0, 7]");
+  if (variant == 5 || variant == 6) ED_TRY(build_two_pass(p, variant == 5, variant == 6, nullptr));
   p->bfp.force_var = variant;
   return ED_OK;
 }

@@ -129,9 +129,112 @@ __global__ void k_row_abs_max(const int32_t* __restrict__ off, const double* __r
   }
 }
 
-static void free_table(SpinTable& t) {
-  cudaFree(t.states); cudaFree(t.energy); cudaFree(t.off); cudaFree(t.idx); cudaFree(t.coef); cudaFree(t.bond);
+static void free_table(const ed_plan_s* p, SpinTable& t) {
+  p->table_free(t.states); p->table_free(t.energy); p->table_free(t.off); p->table_free(t.idx); p->table_free(t.coef);
+  p->table_free(t.bond);
   t = SpinTable();
+}
+
+// Sectors of up to HOST_STATES states per spin get their tables on the host, larger ones by
+// kernels. The tables are a few KB to 2 MB there, and the kernels' chain of launches, copies back
+// and waits costs more than the arithmetic; plan of a half-filled ring, kernels and one
+// allocation per table / host and one allocation (us): 6 sites 1014 / 61, 10 sites 1189 / 110, 14
+// sites (3432 states) 4747 / 840, 15 sites (6435) 2404 / 1863, 16 sites (12870) 887 / 1835.
+constexpr int64_t HOST_STATES = 8192;
+
+// the tables of one spin species with n particles, as the kernels below build them
+static void host_table(const ed_plan_s* p, int n, HostTable* h) {
+  const int N = p->n_sites;
+  const int64_t S = ed_sector_size(N, n);
+  const int nb = (int)p->hop.size();
+  h->states.resize(S);
+  h->energy.resize(S);
+  uint64_t v = n > 0 ? (1ull << n) - 1 : 0;
+  for (int64_t i = 0; i < S; ++i) {
+    h->states[i] = v;
+    double e = 0.0;  // weighted_element: the sites in ascending order
+    for (uint64_t b = v; b; b &= b - 1) e += p->eps[__builtin_ctzll(b)];
+    h->energy[i] = e;
+    if (v) {  // next state with n bits
+      const uint64_t c = v & (~v + 1), r = v + c;
+      v = (((r ^ v) >> 2) / c) | r;
+    }
+  }
+  // index of a state: a table over all 2^N states where that is small, else a binary search
+  std::vector<int32_t> rank;
+  if (N <= 16) {
+    rank.resize((size_t)1 << N);
+    for (int64_t i = 0; i < S; ++i) rank[h->states[i]] = (int32_t)i;
+  }
+  h->off.resize(S + 1);
+  h->off[0] = 0;
+  for (int64_t i = 0; i < S; ++i) {
+    const uint64_t s = h->states[i];
+    for (int b = 0; b < nb; ++b) {
+      const int s1 = p->b1[b], s2 = p->b2[b];
+      if (!(((s >> s1) ^ (s >> s2)) & 1ull)) continue;
+      const uint64_t t = s ^ (1ull << s1) ^ (1ull << s2);
+      h->idx.push_back(rank.empty()
+                           ? (int32_t)(std::lower_bound(h->states.begin(), h->states.end(), t) - h->states.begin())
+                           : rank[t]);
+      h->coef.push_back(hop_sign(s, p->sign_width, s1, s2) < 0 ? -p->hop[b] : p->hop[b]);
+      h->bond.push_back((int16_t)b);
+    }
+    h->off[i + 1] = (int32_t)h->idx.size();
+  }
+}
+
+// a species' tables into the arena; returns their offsets for a second species with the same tables
+struct TableOffsets { size_t v[6]; };
+static TableOffsets place_table(SpinTable& t, const HostTable& h, DeviceArena& a) {
+  TableOffsets o;
+  o.v[0] = a.add(&t.states, h.states.data(), h.states.size() * 8);
+  o.v[1] = a.add(&t.energy, h.energy.data(), h.energy.size() * 8);
+  o.v[2] = a.add(&t.off, h.off.data(), h.off.size() * 4);
+  o.v[3] = a.add(&t.idx, h.idx.data(), h.idx.size() * 4);
+  o.v[4] = a.add(&t.coef, h.coef.data(), h.coef.size() * 8);
+  o.v[5] = a.add(&t.bond, h.bond.data(), h.bond.size() * 2);
+  return o;
+}
+static void share_table(SpinTable& t, const TableOffsets& o, DeviceArena& a) {
+  a.share(&t.states, o.v[0]); a.share(&t.energy, o.v[1]); a.share(&t.off, o.v[2]);
+  a.share(&t.idx, o.v[3]); a.share(&t.coef, o.v[4]); a.share(&t.bond, o.v[5]);
+}
+static void describe_table(SpinTable& t, const HostTable& h) {
+  t.n = (int64_t)h.states.size();
+  t.nnz = (int64_t)h.idx.size();
+  for (int64_t i = 0; i < t.n; ++i) t.max_row = std::max(t.max_row, h.off[i + 1] - h.off[i]);
+}
+// largest row sum of |hop|, and largest |on-site energy|
+static void host_bounds(const HostTable& h, double* row, double* energy) {
+  *row = *energy = 0.0;
+  for (size_t i = 0; i + 1 < h.off.size(); ++i) {
+    double s = 0.0;
+    for (int32_t k = h.off[i]; k < h.off[i + 1]; ++k) s += std::fabs(h.coef[k]);
+    *row = std::max(*row, s);
+    *energy = std::max(*energy, std::fabs(h.energy[i]));
+  }
+}
+
+ed_status download_table(const SpinTable& t, HostTable* h, cudaStream_t s) {
+  h->states.resize(t.n);
+  h->energy.resize(t.n);
+  h->off.resize(t.n + 1);
+  h->idx.resize(t.nnz);
+  h->coef.resize(t.nnz);
+  h->bond.resize(t.nnz);
+  ED_CUDA(cudaMemcpyAsync(h->off.data(), t.off, h->off.size() * 4, cudaMemcpyDeviceToHost, s));
+  if (t.n) {
+    ED_CUDA(cudaMemcpyAsync(h->states.data(), t.states, t.n * 8, cudaMemcpyDeviceToHost, s));
+    ED_CUDA(cudaMemcpyAsync(h->energy.data(), t.energy, t.n * 8, cudaMemcpyDeviceToHost, s));
+  }
+  if (t.nnz) {
+    ED_CUDA(cudaMemcpyAsync(h->idx.data(), t.idx, t.nnz * 4, cudaMemcpyDeviceToHost, s));
+    ED_CUDA(cudaMemcpyAsync(h->coef.data(), t.coef, t.nnz * 8, cudaMemcpyDeviceToHost, s));
+    ED_CUDA(cudaMemcpyAsync(h->bond.data(), t.bond, t.nnz * 2, cudaMemcpyDeviceToHost, s));
+  }
+  ED_CUDA(cudaStreamSynchronize(s));
+  return ED_OK;
 }
 
 static ed_status build_fermion_table(ed_plan_s* p, SpinTable& t, int n, cudaStream_t s) {
@@ -414,10 +517,39 @@ ED_API ed_status ed_plan_create_fermion(const ed_fermion_model* m, int n_up, int
     p->fp.u[i] = m->h_u[i];
     if (m->h_u[i] != p->fp.u0) p->fp.u_uniform = 0;
   }
-  st = build_fermion_table(p, p->up, n_up, s);
-  if (st == ED_OK) st = build_fermion_table(p, p->dn, n_dn, s);
-  if (st == ED_OK) st = finish_bounds(p, s);
-  if (st == ED_OK) st = build_bfp(p, s);
+  auto build = [&]() -> ed_status {
+    DeviceArena arena;
+    HostTable hu, hd_own;
+    const bool same = n_up == n_dn;
+    const HostTable& hd = same ? hu : hd_own;
+    if (std::max(nu, nd) <= HOST_STATES) {
+      host_table(p, n_up, &hu);
+      if (!same) host_table(p, n_dn, &hd_own);
+      describe_table(p->up, hu);
+      describe_table(p->dn, hd);
+      double ru, rd, eu, edn, su = 0.0;
+      host_bounds(hu, &ru, &eu);
+      host_bounds(hd, &rd, &edn);
+      for (double v : p->u) su += std::fabs(v);
+      p->hnorm_bound = (eu + edn + su) + ru + rd;
+      const TableOffsets o = place_table(p->up, hu, arena);
+      if (same) share_table(p->dn, o, arena);
+      else place_table(p->dn, hd, arena);
+      if (bfp_possible(p)) ED_TRY(build_bfp(p, hu, hd, arena));
+    } else {
+      ED_TRY(build_fermion_table(p, p->up, n_up, s));
+      ED_TRY(build_fermion_table(p, p->dn, n_dn, s));
+      ED_TRY(finish_bounds(p, s));
+      if (bfp_possible(p)) {
+        ED_TRY(download_table(p->up, &hu, s));
+        if (!same) ED_TRY(download_table(p->dn, &hd_own, s));
+        ED_TRY(build_bfp(p, hu, hd, arena));
+      }
+    }
+    ED_TRY(arena.commit(&p->arena, &p->arena_bytes, s));
+    return build_default_two_pass(p, s);
+  };
+  st = build();
   if (st != ED_OK) { ed_plan_destroy(p); return st; }
   *out = p;
   return ED_OK;
@@ -492,10 +624,11 @@ ED_API ed_status ed_plan_destroy(ed_plan p) {
   int prev = -1;
   cudaGetDevice(&prev);
   if (p->device >= 0 && prev != p->device) cudaSetDevice(p->device);
-  free_table(p->up);
-  free_table(p->dn);
+  free_table(p, p->up);
+  free_table(p, p->dn);
   free_bfp(p);
   cudaFree(p->spin_diag);
+  cudaFree(p->arena);
   if (prev >= 0 && prev != p->device) cudaSetDevice(prev);
   delete p;
   return ED_OK;

@@ -8,11 +8,51 @@
 // Spin sectors keep one table over the states plus the precomputed diagonal.
 #pragma once
 
+#include <string.h>
+
+#include <algorithm>
+#include <utility>
 #include <vector>
 
 #include "ed_common.cuh"
 
 namespace ed {
+
+// One device allocation that holds many small tables: add() places a copy of a host array (256
+// byte aligned) and commit() allocates, copies everything in one transfer, sets the pointers and
+// waits. A plan has about 25 tables of a few KB; allocated, copied and freed one by one they were
+// most of the 1.2 ms that a small sector's plan took.
+struct DeviceArena {
+  std::vector<unsigned char> host;
+  std::vector<std::pair<void**, size_t>> fix;
+  template <class T>
+  size_t add(T** dst, const void* src, size_t bytes) {
+    const size_t off = host.size();
+    host.resize(off + (std::max<size_t>(bytes, 8) + 255) / 256 * 256);
+    if (bytes) memcpy(host.data() + off, src, bytes);
+    fix.emplace_back((void**)dst, off);
+    return off;
+  }
+  template <class T>
+  void share(T** dst, size_t off) { fix.emplace_back((void**)dst, off); }
+  ed_status commit(unsigned char** dev, size_t* size, cudaStream_t s) {
+    if (host.empty()) return ED_OK;
+    ED_CUDA(cudaMalloc((void**)dev, host.size()));
+    *size = host.size();
+    for (auto& f : fix) *f.first = *dev + f.second;
+    ED_CUDA(cudaMemcpyAsync(*dev, host.data(), host.size(), cudaMemcpyHostToDevice, s));
+    ED_CUDA(cudaStreamSynchronize(s));  // the tables may be read from any stream
+    return ED_OK;
+  }
+};
+
+// host copy of one spin species' tables (as SpinTable)
+struct HostTable {
+  std::vector<uint64_t> states;
+  std::vector<double> energy, coef;
+  std::vector<int32_t> off, idx;
+  std::vector<int16_t> bond;
+};
 
 struct SpinTable {
   int64_t n = 0;              // number of states of this spin species
@@ -146,6 +186,7 @@ struct BfpTables {
   DnCompactTables dc;
   long wait_limit = 0;          // polls of a first bulk-copy wait before giving up (0: default)
   int force_var = 0;            // matvec variant chosen for this plan (0: automatic)
+  bool sw_tried = false, sp_tried = false;  // the tables of variants 5 / 6 were asked for
 };
 
 }  // namespace ed
@@ -171,6 +212,13 @@ struct ed_plan_s {
   double* spin_diag = nullptr;  // spin: [D]
   ed::DeviceContext* ctx = nullptr;
   ed::BfpTables bfp;
+  // tables that live in one allocation (DeviceArena)
+  unsigned char* arena = nullptr;
+  size_t arena_bytes = 0;
+  // frees a table that is not part of the arena
+  void table_free(void* q) const {
+    if (!((unsigned char*)q >= arena && (unsigned char*)q < arena + arena_bytes)) cudaFree(q);
+  }
 };
 
 namespace ed {
@@ -179,8 +227,14 @@ ed_status check_plan(const ed_plan_s* p);
 // y = H x for nvec vectors (leading dimension ld); skipped when *stop != 0 (stop may be null).
 ed_status matvec_f64(const ed_plan_s* p, const double* x, double* y, int64_t nvec, int64_t ld, cudaStream_t s,
                      const int* stop = nullptr);
-// Builds p->bfp when the sector qualifies (called at plan creation; synchronous).
-ed_status build_bfp(ed_plan_s* p, cudaStream_t s);
+// Builds p->bfp when the sector qualifies (called at plan creation); its tables go into `arena`.
+bool bfp_possible(const ed_plan_s* p);
+ed_status build_bfp(ed_plan_s* p, const HostTable& hu, const HostTable& hd, DeviceArena& arena);
+// the tables of the two-pass variants 5 and 6 that the plan's matvec may take (synchronous)
+ed_status build_two_pass(ed_plan_s* p, bool sweep, bool stripe, cudaStream_t s);
+ed_status build_default_two_pass(ed_plan_s* p, cudaStream_t s);
+// host copy of a species' device tables (synchronous)
+ed_status download_table(const SpinTable& t, HostTable* h, cudaStream_t s);
 void free_bfp(ed_plan_s* p);
 // fixed-point Lanczos (ed_bfp.cu)
 size_t bfp_workspace_bytes(const ed_plan_s* p, int K, bool store);

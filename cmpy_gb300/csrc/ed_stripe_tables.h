@@ -35,9 +35,10 @@ struct StripeSide {
 // coefficients are no hops) in increasing (pairs, - pairs) order, ties by original index, and
 // the hop lists of the renumbered targets: the record slots of the + partners, then of the -
 // partners, each segment padded to whole pairs with the zero record (record n). False when a
-// target needs more than ST_PMAX pairs or n is too large for 16-bit slots.
+// target needs more than ST_PMAX pairs or n is too large for 16-bit slots. lists = false: the
+// order and the pair counts alone.
 static bool stripe_order(int64_t n, const std::vector<int32_t>& off, const std::vector<int32_t>& idx,
-                         const std::vector<double>& coef, StripeSide* out) {
+                         const std::vector<double>& coef, StripeSide* out, bool lists = true) {
   if (n < 1 || 2 * n + 1 >= 65536) return false;
   std::vector<int> pp(n), pn(n);
   for (int64_t v = 0; v < n; ++v) {
@@ -62,9 +63,11 @@ static bool stripe_order(int64_t n, const std::vector<int32_t>& off, const std::
   int pmax = 0;
   for (int64_t v = 0; v < n; ++v) pmax = std::max(pmax, pp[v] + pn[v]);
   out->pmax = pmax;
+  out->meta.resize(n);
+  for (int64_t i = 0; i < n; ++i) out->meta[i] = (uint16_t)(pp[perm[i]] | (pn[perm[i]] << 8));
+  if (!lists) return true;
   const uint32_t zero = stripe_slot(n);
   out->lst.assign((size_t)std::max(pmax, 1) * n, zero | (zero << 16));
-  out->meta.assign(n, 0);
   std::vector<uint32_t> seg;
   for (int64_t i = 0; i < n; ++i) {
     const int64_t v = perm[i];
@@ -76,7 +79,6 @@ static bool stripe_order(int64_t n, const std::vector<int32_t>& off, const std::
       if (seg.size() % 2) seg.push_back(zero);
       for (size_t e = 0; e < seg.size(); e += 2) out->lst[(size_t)p++ * n + i] = seg[e] | (seg[e + 1] << 16);
     }
-    out->meta[i] = (uint16_t)(pp[v] | (pn[v] << 8));
   }
   return true;
 }
