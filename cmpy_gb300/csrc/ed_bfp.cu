@@ -538,11 +538,10 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
       "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(pol)
       : "memory");
 }
-// read-only data (X is not written while the kernel runs), so the asm is not volatile: the
-// compiler may batch these loads
+// (volatile: the compiler must not move the load above the test that keeps its address in range)
 __device__ __forceinline__ int64_t ld_keep(const int64_t* p, uint64_t pol) {
   int64_t v;
-  asm("ld.global.nc.L2::cache_hint.s64 %0, [%1], %2;" : "=l"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.nc.L2::cache_hint.s64 %0, [%1], %2;" : "=l"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ void st_stream(int64_t* p, int64_t v, uint64_t pol) {
