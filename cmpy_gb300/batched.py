@@ -92,7 +92,7 @@ class Batch:
             return hit
         # size the workspace for the largest candidate grid
         best = 0
-        for t, ps, cs in ((128, 4, 1), (256, 2, 1), (256, 4, 1), (512, 1, 1), (512, 2, 1), (1024, 1, 1),
+        for t, ps, cs in ((256, 2, 1), (256, 3, 1), (256, 4, 1), (512, 1, 1), (512, 2, 1), (1024, 1, 1),
                           (512, 2, 2), (1024, 1, 2), (512, 2, 4), (1024, 1, 4), (512, 2, 8), (1024, 1, 8)):
             nb = C.c_size_t()
             N.check(N.lib().ed_batch_workspace(self._h, int(tune_steps), t, ps, cs, C.byref(nb)))
@@ -107,6 +107,31 @@ class Batch:
         self.threads, self.ctas_per_sm, self.cluster_size = int(th.value), int(ps.value), int(cs.value)
         _tune_cache[key] = (self.threads, self.ctas_per_sm, self.cluster_size, float(ms.value))
         return _tune_cache[key]
+
+    def _starts(self, starts):
+        """Device array of the start vectors' pointers (None: seeded starts)."""
+        if starts is None:
+            return None
+        st = [E._as_dev_f64(x).reshape(-1) for x in starts]
+        if [x.numel() for x in st] != self.dims:
+            raise ValueError("start vectors must match the problem dimensions")
+        self._starts_keep = st
+        self._starts_dev = torch.as_tensor(np.array([x.data_ptr() for x in st], dtype=np.int64)).to(E.device())
+        return self._starts_dev.data_ptr()
+
+    def coeffs(self, max_steps: int, starts: Sequence[torch.Tensor] | None = None, seed: int = 0):
+        """Lanczos coefficients of every problem (alpha [n, K], beta [n, K+1], steps [n]), no tests,
+        energies or vectors. Asynchronous."""
+        K = int(max_steps)
+        ws = self.workspace(K, self.threads, self.ctas_per_sm, self.cluster_size)
+        dev = E.device()
+        alpha = torch.empty((self.n, K), dtype=torch.float64, device=dev)
+        beta = torch.empty((self.n, K + 1), dtype=torch.float64, device=dev)
+        steps = torch.empty(self.n, dtype=torch.int32, device=dev)
+        N.check(N.lib().ed_batch_lanczos_coeffs(
+            self._h, K, int(seed), self._starts(starts), N.ptr(ws), ws.numel(), N.ptr(alpha), N.ptr(beta),
+            N.ptr(steps), int(self.threads), int(self.ctas_per_sm), int(self.cluster_size), E._stream()))
+        return alpha, beta, steps
 
     def lanczos(self, max_steps: int = 300, tol: float = 1e-12, check_every: int = 10, seed: int = 0,
                 starts: Sequence[torch.Tensor] | None = None, want_vector: bool = False,
@@ -125,14 +150,7 @@ class Batch:
                 self._voff = torch.as_tensor(offs).to(E.device())
                 self._vbuf = vbuf
             out = BatchResult(e, s, r, a, b, vecs)
-        starts_ptr = None
-        if starts is not None:
-            st = [E._as_dev_f64(x).reshape(-1) for x in starts]
-            if [x.numel() for x in st] != self.dims:
-                raise ValueError("start vectors must match the problem dimensions")
-            self._starts_keep = st
-            self._starts_dev = torch.as_tensor(np.array([x.data_ptr() for x in st], dtype=np.int64)).to(E.device())
-            starts_ptr = self._starts_dev.data_ptr()
+        starts_ptr = self._starts(starts)
         N.check(N.lib().ed_batch_lanczos(
             self._h, K, float(tol), int(check_every), int(seed), starts_ptr, int(bool(want_vector)), N.ptr(ws),
             ws.numel(), N.ptr(out.alpha), N.ptr(out.beta), N.ptr(out.energy), N.ptr(out.residual), N.ptr(out.steps),
@@ -210,8 +228,8 @@ def greens_functions_batched(models, sectors, z, pos: int = 0, sigma: int = 1, g
         b = Batch(tplans)
         if tune:
             b.tune(min(40, gf_levels))
-        res = b.lanczos(max_steps=gf_levels, tol=0.0, check_every=0, starts=starts)
-        part = batch_cf(res, gs.energy[idx], sign, zt)
+        alpha, beta, steps = b.coeffs(gf_levels, starts)
+        part = batch_cf(BatchResult(None, steps, None, alpha, beta, None), gs.energy[idx], sign, zt)
         g[idx] += part
     return gs.energy, g
 

@@ -1471,13 +1471,20 @@ ed_status build_bfp(ed_plan_s* p, const HostTable& hu, const HostTable& hd, Devi
       if (ucoef[k] < 0.0) bidx.push_back(uidx[k]);
     bnpos[r] = npos;
     max_up = std::max(max_up, (int)(bidx.size() - boff[r]));
+    B.quads[0] = std::max(B.quads[0], (npos + 3) / 4);
+    B.quads[1] = std::max(B.quads[1], ((int)(bidx.size() - boff[r]) - npos + 3) / 4);
   }
   boff[nu] = (int32_t)bidx.size();
   int max_dn = 0;
   for (int64_t c = 0; c < nd; ++c) {
-    int n = 0;
-    for (int32_t k = doff[c]; k < doff[c + 1]; ++k) n += (dcoef[k] != 0.0);
+    int n = 0, np = 0;
+    for (int32_t k = doff[c]; k < doff[c + 1]; ++k) {
+      n += (dcoef[k] != 0.0);
+      np += (dcoef[k] > 0.0);
+    }
     max_dn = std::max(max_dn, n);
+    B.quads[2] = std::max(B.quads[2], (np + 3) / 4);
+    B.quads[3] = std::max(B.quads[3], (n - np + 3) / 4);
   }
   std::vector<uint16_t> tab((size_t)std::max(max_dn, 1) * nd, (uint16_t)(2 * nd));
   for (int64_t c = 0; c < nd; ++c) {

@@ -158,6 +158,7 @@ struct BfpTables {
   int64_t* e_up_fx = nullptr;  // diag64: [nu]
   int64_t* e_dn_fx = nullptr;  // diag64: [nd]
   int max_dn = 0;         // dn table entries per column (padded)
+  int quads[4] = {};      // largest numbers of up +, up -, dn +, dn - partners of a state, in fours
   int vec2 = 0;           // num_dn even: 128-bit row loads
   // up: per target row, neighbours with + sign first, then - sign
   int32_t* up_off = nullptr;   // [nu+1]

@@ -349,6 +349,13 @@ ED_API ed_status ed_batch_lanczos(ed_batch batch, int max_steps, double tol, int
                                   double* d_energy, double* d_residual, int32_t* d_steps,
                                   double* d_vecs, const int64_t* d_vec_offsets, int threads,
                                   int ctas_per_sm, int cluster_size, ed_stream_t stream);
+/* The Lanczos coefficients alone: ed_batch_lanczos without convergence tests, energies, residuals and
+ * vectors (the runs of continued fractions). */
+ED_API ed_status ed_batch_lanczos_coeffs(ed_batch b, int max_steps, uint64_t seed, const double* const* d_starts,
+                                         void* d_work, size_t work_bytes, double* d_alpha, double* d_beta,
+                                         int32_t* d_steps, int threads, int ctas_per_sm, int cluster_size,
+                                         ed_stream_t stream);
+
 /* Launch configuration: threads per CTA (128, 256, 512, 1024), CTAs per SM, and the
  * thread-block cluster size per problem (1, or 2/4/8 with 512 or 1024 threads: the cluster's
  * CTAs share each problem's vectors and exchange their partial sums through distributed
