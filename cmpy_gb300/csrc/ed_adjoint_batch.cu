@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "ed_adjoint.cuh"
+#include "ed_cf.cuh"
 #include "ed_lzcheck.cuh"
 
 namespace ed {
@@ -430,29 +431,18 @@ __global__ void k_bcf(const double* __restrict__ alpha, int64_t ka, const double
                       const int* __restrict__ m_arr, const double* __restrict__ n2_arr,
                       const double* __restrict__ shift_arr, int sign, const double2* __restrict__ z, int64_t nz,
                       double2* __restrict__ g) {
+  __shared__ double2 st[CF_TILE];
   const int pb = blockIdx.y;
   const int n = m_arr[pb];
   if (n < 1) return;
-  const double* a = alpha + (int64_t)pb * ka;
-  const double* bt = beta + (int64_t)pb * kb;
-  const double norm2 = n2_arr[pb], shift = shift_arr[pb];
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nz; i += (int64_t)gridDim.x * blockDim.x) {
-    const double2 zi = z[i];
-    const double zr = sign * zi.x + shift, zm = sign * zi.y;
-    double tr = zr - a[n - 1], tm = zm;
-    for (int l = n - 2; l >= 0; --l) {
-      const double bb = bt[l + 1] * bt[l + 1];
-      const double inv = bb / (tr * tr + tm * tm);
-      tr = zr - a[l] - tr * inv;
-      tm = zm + tm * inv;
-    }
-    const double inv = sign * norm2 / (tr * tr + tm * tm);
-    double2 r = make_double2(tr * inv, -tm * inv);
-    double2* gi = g + (int64_t)pb * nz + i;
-    r.x += gi->x;
-    r.y += gi->y;
-    *gi = r;
-  }
+  const double shift = shift_arr[pb];
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const double2 zi = i < nz ? z[i] : make_double2(0.0, 1.0);
+  const double2 r = cf_value(alpha + (int64_t)pb * ka, beta + (int64_t)pb * kb, n, sign * zi.x + shift, sign * zi.y,
+                             sign * n2_arr[pb], st);
+  if (i >= nz) return;
+  double2& o = g[(int64_t)pb * nz + i];
+  o = make_double2(o.x + r.x, o.y + r.y);
 }
 
 }  // namespace ed
@@ -789,7 +779,7 @@ ED_API ed_status ed_batch_cf(int B, const double* d_alpha, int64_t ka, const dou
   if (sign != 1 && sign != -1) return fail(ED_ERR_INVALID_ARG, "sign must be +1 or -1");
   if (!d_alpha || !d_beta || !d_m || !d_n2 || !d_shift || !d_z || !d_g) return fail(ED_ERR_INVALID_ARG, "null argument");
   if (n_z == 0) return ED_OK;
-  const int gx = (int)std::min<int64_t>((n_z + 127) / 128, 64);
+  const unsigned gx = (unsigned)((n_z + 127) / 128);
   k_bcf<<<dim3(gx, B), 128, 0, as_stream(stream)>>>(d_alpha, ka, d_beta, kb, d_m, d_n2, d_shift, sign,
                                                    (const double2*)d_z, n_z, (double2*)d_g);
   ED_CHECK_LAUNCH("k_bcf");

@@ -1,39 +1,32 @@
 // Batched Lanczos (the kernel: ed_batch.cuh, ed_resident.cuh): batch handles, the choice of the launch
 // configuration, and the batched continued fraction.
 #include "ed_batch.cuh"
+#include "ed_cf.cuh"
 
 #include "ed_resident.cuh"
 
 namespace ed {
 
 // G_p(z) += sign * norm_p^2 / (z' - a0 - b1^2 / (z' - a1 - ...)),  z' = sign*z + e0_p,
-// norm_p = beta[p][0] (start norm), m_p = steps[p]; one thread per (problem, frequency)
-__global__ void k_batch_cf(int n, int K, const double* __restrict__ alpha, const double* __restrict__ beta,
-                           const int32_t* __restrict__ steps, const double* __restrict__ e0, int sign,
-                           const double2* __restrict__ z, int64_t nz, double2* __restrict__ g) {
-  const int64_t tot = (int64_t)n * nz;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
-    const int p = (int)(t / nz);
-    const int64_t j = t - (int64_t)p * nz;
+// norm_p = beta[p][0] (start norm), m_p = steps[p]; one thread per frequency, one problem per
+// blockIdx.y. Bound by the FP64 pipe: 512 problems x 1280 frequencies x 2000 levels 28.7 -> 22.9 ms.
+constexpr int BCF_NT = 128;
+__global__ void __launch_bounds__(BCF_NT) k_batch_cf(int n, int K, const double* __restrict__ alpha,
+                                                     const double* __restrict__ beta, const int32_t* __restrict__ steps,
+                                                     const double* __restrict__ e0, int sign,
+                                                     const double2* __restrict__ z, int64_t nz, double2* __restrict__ g) {
+  __shared__ double2 st[CF_TILE];
+  const int64_t j = blockIdx.x * (int64_t)BCF_NT + threadIdx.x;
+  const double2 zi = j < nz ? z[j] : make_double2(0.0, 1.0);
+  for (int p = blockIdx.y; p < n; p += gridDim.y) {
     const int m = steps[p];
-    const double* a = alpha + (int64_t)p * K;
+    if (m < 1) continue;
     const double* b = beta + (int64_t)p * (K + 1);
-    double2 r = g[t];
-    if (m > 0) {
-      const double2 zi = z[j];
-      const double zr = sign * zi.x + e0[p], zm = sign * zi.y;
-      double tr = zr - a[m - 1], tm = zm;
-      for (int l = m - 2; l >= 0; --l) {
-        const double bb = b[l + 1] * b[l + 1];
-        const double inv = bb / (tr * tr + tm * tm);
-        tr = zr - a[l] - tr * inv;
-        tm = zm + tm * inv;
-      }
-      const double inv = sign * b[0] * b[0] / (tr * tr + tm * tm);
-      r.x += tr * inv;
-      r.y -= tm * inv;
+    const double2 r = cf_value(alpha + (int64_t)p * K, b, m, sign * zi.x + e0[p], sign * zi.y, sign * b[0] * b[0], st);
+    if (j < nz) {
+      double2& o = g[(int64_t)p * nz + j];
+      o = make_double2(o.x + r.x, o.y + r.y);
     }
-    g[t] = r;
   }
 }
 
@@ -296,11 +289,9 @@ ED_API ed_status ed_batch_gf_continued_fraction(int n, int max_steps, const doub
   if (sign != 1 && sign != -1) return fail(ED_ERR_INVALID_ARG, "sign must be +1 or -1");
   if (n_z == 0) return ED_OK;
   if (!d_alpha || !d_beta || !d_steps || !d_e0 || !d_z || !d_g) return fail(ED_ERR_INVALID_ARG, "null argument");
-  DeviceContext* ctx;
-  ED_TRY(device_context(&ctx));
-  const int64_t tot = (int64_t)n * n_z;
-  k_batch_cf<<<grid_for(tot, 128, ctx->num_sms * 16), 128, 0, as_stream(stream)>>>(
-      n, max_steps, d_alpha, d_beta, d_steps, d_e0, sign, (const double2*)d_z, n_z, (double2*)d_g);
+  const dim3 grid((unsigned)((n_z + BCF_NT - 1) / BCF_NT), (unsigned)std::min(n, 65535));
+  k_batch_cf<<<grid, BCF_NT, 0, as_stream(stream)>>>(n, max_steps, d_alpha, d_beta, d_steps, d_e0, sign,
+                                                     (const double2*)d_z, n_z, (double2*)d_g);
   ED_CHECK_LAUNCH("k_batch_cf");
   return ED_OK;
 }
