@@ -1695,13 +1695,17 @@ static int v3_threads(const ed_plan_s* p) {
 // one stage), else 1; 6 (two-pass stripes in a renumbered basis, ed_stripe.cuh), 5 and 3 when
 // forced. Rows must have an even length (16-byte row copies). CMPY_ED_MATVEC=1..7 or
 // ed_plan_set_matvec_variant forces a variant when possible.
-static int matvec_variant(const ed_plan_s* p) {
+int forced_variant(const ed_plan_s* p) {
   static int env_forced = -1;
   if (env_forced < 0) {
     const char* e = getenv("CMPY_ED_MATVEC");
     env_forced = e ? atoi(e) : 0;
   }
-  const int forced = p->bfp.force_var > 0 ? p->bfp.force_var : env_forced;
+  return p->bfp.force_var > 0 ? p->bfp.force_var : env_forced;
+}
+
+static int matvec_variant(const ed_plan_s* p) {
+  const int forced = forced_variant(p);
   const size_t optin = (size_t)p->ctx->smem_optin;
   const bool v2_ok = p->bfp.vec2 && v2_smem(p) + MV2_STATIC_SMEM <= optin && p->num_up >= 1;
   // list entries are int32 element offsets u * nd: the vector must have fewer than 2^31 elements
@@ -2124,12 +2128,14 @@ ed_status bfp_lanczos(const ed_plan_s* p, const ed_lanczos_params* prm, const do
   const int64_t D = p->dim;
   const bool store = prm->want_vector != 0;
   BfpRun r = bfp_bind(p, work, K, store);
-  const int32_t *pu, *pd;
-  (void)matvec_perms(p, &pu, &pd);
+  // a small sector's run is one launch (per-matvec times need the launched steps)
+  const bool resident = !prm->profile && resident_fits(p);
+  const int32_t *pu = nullptr, *pd = nullptr;
+  if (!resident) (void)matvec_perms(p, &pu, &pd);
   ED_CUDA(cudaMemsetAsync(r.st, 0, sizeof(BfpState), s));
   ED_CUDA(cudaMemsetAsync(alpha, 0, K * sizeof(double), s));
   ED_CUDA(cudaMemsetAsync(beta, 0, (K + 1) * sizeof(double), s));
-  ED_TRY(bfp_start(p, r, v0_dev, beta, s, pu, pd));
+  if (!resident) ED_TRY(bfp_start(p, r, v0_dev, beta, s, pu, pd));
   const int Km = (int)std::min<int64_t>(K, D);
   std::vector<cudaEvent_t> ev;
   if (prm->profile) {
@@ -2139,10 +2145,15 @@ ed_status bfp_lanczos(const ed_plan_s* p, const ed_lanczos_params* prm, const do
   // convergence tests on a side stream and the final eigenpair, on the device (ed_lzcheck.cuh)
   const bool checks = prm->check_every > 0 && prm->tol > 0.0;
   SideChecks chk;
-  ED_TRY(chk.init(checks ? Km / prm->check_every + 1 : 0));
+  ED_TRY(chk.init(checks && !resident ? Km / prm->check_every + 1 : 0));
   ED_CUDA(cudaMemsetAsync(r.tri, 0, sizeof(TriResult), s));
   int launched = 0;
-  for (int k = 0; k < Km; ++k) {
+  if (resident) {
+    ED_TRY(resident_run(p, K, prm->tol, checks ? prm->check_every : 0, v0_dev, alpha, beta, &r.st->energy, 0, r.v.eR,
+                        store ? r.v.R : nullptr, r.c, r.work, &r.st->stop, &r.st->steps, &r.st->status, r.tri, s));
+    launched = Km;
+  }
+  for (int k = launched; k < Km; ++k) {
     if (checks && chk.stopped()) break;
     if (prm->profile) ED_CUDA(cudaEventRecord(ev[2 * k], s));
     const BfpFuse fz = bfp_fuse(p, r, k, alpha, beta);
@@ -2177,6 +2188,8 @@ ed_status bfp_lanczos(const ed_plan_s* p, const ed_lanczos_params* prm, const do
   ED_CUDA(cudaMemcpyAsync(&ht, r.tri, sizeof(TriResult), cudaMemcpyDeviceToHost, s));
   ED_CUDA(cudaStreamSynchronize(s));
   if (hs.status == DEV_TIMEOUT) return fail(ED_ERR_TIMEOUT, "fixed-point matvec: a bounded wait for a row copy ran out");
+  if (hs.status == DEV_NONFINITE) return fail(ED_ERR_NONFINITE, "start vector is not finite");
+  if (hs.status == RES_ZERO_START) return fail(ED_ERR_ZERO_VECTOR, "start vector has zero norm");
   const int m = ht.m_final;
   res->energy = ht.energy;
   res->residual = ht.residual;
@@ -2206,9 +2219,11 @@ struct BfpCoeffRun {
   double *alpha, *beta;
   int Km = 0;
   bool empty = false;  // zero start vector: an empty Krylov space
+  bool resident = false;  // the whole run is one launch
 };
 
-// memsets, the start vector's finiteness and zero test (synchronous on s), R_0 and beta_0
+// memsets, the start vector's finiteness and zero test (synchronous on s), R_0 and beta_0; or the whole
+// run's launch
 static ed_status bfp_coeffs_begin(const ed_plan_s* p, int K, const double* start, void* work, double* alpha,
                                   double* beta, cudaStream_t s, BfpCoeffRun* run) {
   const int64_t D = p->dim;
@@ -2220,6 +2235,11 @@ static ed_status bfp_coeffs_begin(const ed_plan_s* p, int K, const double* start
   ED_CUDA(cudaMemsetAsync(r.st, 0, sizeof(BfpState), s));
   ED_CUDA(cudaMemsetAsync(alpha, 0, K * sizeof(double), s));
   ED_CUDA(cudaMemsetAsync(beta, 0, (K + 1) * sizeof(double), s));
+  if (resident_fits(p)) {
+    run->resident = true;
+    return resident_run(p, K, 0.0, 0, start, alpha, beta, &r.st->energy, 1, r.v.eR, nullptr, r.c, r.work, &r.st->stop,
+                        &r.st->steps, &r.st->status, nullptr, s);
+  }
   {
     const int gs = grid_for(D, 256, p->ctx->num_sms * 8);
     unsigned long long* mxb = (unsigned long long*)(r.misc + 8);
@@ -2251,6 +2271,14 @@ static ed_status bfp_coeffs_end(BfpCoeffRun& run, int* steps, double* norm, cuda
     return ED_OK;
   }
   BfpState hs;
+  if (run.resident) {
+    ED_CUDA(cudaMemcpyAsync(&hs, run.r.st, sizeof(BfpState), cudaMemcpyDeviceToHost, s));
+    ED_CUDA(cudaStreamSynchronize(s));
+    if (hs.status == DEV_NONFINITE) return fail(ED_ERR_NONFINITE, "start vector is not finite");
+    *steps = hs.steps;  // (0 for a zero start vector)
+    *norm = hs.status == RES_ZERO_START ? 0.0 : hs.energy;
+    return ED_OK;
+  }
   double b0 = 0.0;
   ED_CUDA(cudaMemcpyAsync(&hs, run.r.st, sizeof(BfpState), cudaMemcpyDeviceToHost, s));
   ED_CUDA(cudaMemcpyAsync(&b0, run.beta, sizeof(double), cudaMemcpyDeviceToHost, s));

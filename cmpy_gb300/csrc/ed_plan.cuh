@@ -247,4 +247,14 @@ ed_status bfp_lanczos_coeffs_multi(int n, const ed_plan_s* const* plans, int K, 
                                    double* norms, cudaStream_t s);
 ed_status bfp_lanczos_coeffs(const ed_plan_s* p, int K, const double* start, void* work, double* alpha,
                              double* beta, int* steps, double* norm, cudaStream_t s);
+// a run of a small sector in one launch (ed_resident_run.cu): whether p's runs take it; the run itself
+// (alpha, beta, exps, c: K + 1 values; store [K][dim] or null; work 5 K; the state words are zero before.
+// status: DEV_NONFINITE or RES_ZERO_START for such a start; zero_beta0: beta[0] = 0, the norm only in *norm)
+struct TriResult;
+int forced_variant(const ed_plan_s* p);  // the matvec kernel asked for by the plan or the environment (0: none)
+constexpr int RES_ZERO_START = 16;
+bool resident_fits(const ed_plan_s* p);
+ed_status resident_run(const ed_plan_s* p, int K, double tol, int check_every, const double* start, double* alpha,
+                       double* beta, double* norm, int zero_beta0, int32_t* exps, int64_t* store, double* c,
+                       double* work, int* stop, int* steps, int* status, TriResult* tri, cudaStream_t s);
 }  // namespace ed

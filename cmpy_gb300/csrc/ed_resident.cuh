@@ -301,6 +301,8 @@ struct ResShared {
   unsigned long long mk, mp;
   int ek, ep;
   double lo, hi;                   // bracket of the lowest eigenvalue (res_test)
+  double e;                        // the last careful solution: lowest eigenvalue of T_me, its vector in c
+  int me;
   int cnt[128];
 };
 
@@ -605,7 +607,7 @@ struct ResRun {
   uint64_t* acc_lo;
   int64_t* acc_hi;
   int64_t* store;       // [K][D] or null
-};
+};  // (alpha null: this CTA of a cluster records nothing)
 template <int NT, int CS, int MODE, bool DIAG64>
 static __device__ __noinline__ int res_recurrence(const BatchProblem& P, const ResTables T, const ResRun& io, ResShared& s) {
   extern __shared__ __align__(16) unsigned char res_sm[];
@@ -613,7 +615,8 @@ static __device__ __noinline__ int res_recurrence(const BatchProblem& P, const R
   int64_t* const Rp = MODE == RES_ALL ? (int64_t*)(res_sm + T.rp) : io.Rp;
   int64_t* const W = MODE == RES_ALL ? (int64_t*)(res_sm + T.w) : io.W;
   constexpr int NC = NT - 32;  // threads that own elements; the last warp does the scalars
-  const bool pass2 = io.Ck != nullptr;
+  const bool pass2 = io.Ck != nullptr, rec = !pass2 && io.alpha != nullptr;
+  const bool rk0 = CS == 1 || io.rk == 0;
   const int lane = threadIdx.x & 31;
   const bool scalar = (int)(threadIdx.x >> 5) == NT / 32 - 1;
   const int64_t D = P.D, i0 = scalar ? D : (int64_t)io.rk * NC + threadIdx.x, st = (int64_t)CS * NC;
@@ -645,7 +648,7 @@ static __device__ __noinline__ int res_recurrence(const BatchProblem& P, const R
   if constexpr (CS > 1) res_collect<CS>(s, 0, &tot, &tmax);
   const double mx0 = __longlong_as_double((long long)tmax);
   if (tmax == 0 || tmax >= 0x7FF0000000000000ull) {  // the same in every thread of the cluster
-    if (threadIdx.x == 0 && !pass2) beta[0] = tmax == 0 ? 0.0 : nan("");
+    if (threadIdx.x == 0 && rec) beta[0] = tmax == 0 ? 0.0 : nan("");
     csync<CS>();
     return 0;
   }
@@ -669,6 +672,7 @@ static __device__ __noinline__ int res_recurrence(const BatchProblem& P, const R
   if (threadIdx.x == 0) {
     s.stop = 0;
     s.m = 0;
+    s.me = 0;
     s.lo = 0.0;
     s.hi = 0.0;
     s.bk = 0.0;
@@ -688,9 +692,11 @@ static __device__ __noinline__ int res_recurrence(const BatchProblem& P, const R
       s.bk = bk;
       s.mp = s.mk;
       s.mk = tmax;
-      if (!pass2) {
+      if (rec) {
         beta[k] = bk;
         io.exps[k] = s.ek;
+      }
+      if (!pass2) {
         // the new residual vanishes relative to the scale of T (beta[0] holds the start-vector norm,
         // not an entry of T)
         if (k > 0 && (!(bk > 1e-13 * s.row) || tmax == 0)) {
@@ -778,7 +784,7 @@ static __device__ __noinline__ int res_recurrence(const BatchProblem& P, const R
     __syncthreads();
     if (scalar) {
       if (lane == 0) {
-        if (!pass2) alpha[k] = a_k;
+        if (rec) alpha[k] = a_k;
         s.row = fabs(a_k) + (k > 0 ? s.bk : 0.0) + 1e-300;
       }
       __syncwarp();
@@ -819,17 +825,29 @@ static __device__ __noinline__ int res_recurrence(const BatchProblem& P, const R
       pending = false;
       __syncthreads();
       if (s.stop) break;
-      // every CTA of the cluster tests the same tridiagonal (same data, same result); a pass is
-      // confirmed by the careful solver
-      if (res_test(alpha, beta, k + 1, io.work, s) <= 2.0 * io.tol) {
+      // the first CTA of a cluster tests; a pass is confirmed by the careful solver
+      if (rk0 && res_test(alpha, beta, k + 1, io.work, s) <= 2.0 * io.tol) {
         const double e = res_tridiag(alpha, beta, k + 1, io.c, io.work, s.lo, s.hi);
-        if (threadIdx.x == 0 && fabs(beta[k + 1] * io.c[k]) <= io.tol * fmax(1.0, fabs(e))) {
-          s.stop = 1;
+        if (threadIdx.x == 0) {
+          s.e = e;
+          s.me = k + 1;
+          if (fabs(beta[k + 1] * io.c[k]) <= io.tol * fmax(1.0, fabs(e))) {
+            s.stop = 1;
+            s.m = k + 1;
+          }
+        }
+        __syncthreads();
+      }
+      if constexpr (CS > 1) {
+        csync<CS>();  // (s.stop of the first CTA does not change again before the next cluster barrier)
+        const int stop0 = *cg::this_cluster().map_shared_rank(&s.stop, 0);
+        if (threadIdx.x == 0 && !rk0) {
+          s.stop = stop0;
           s.m = k + 1;
         }
         __syncthreads();
-        if (s.stop) break;
       }
+      if (s.stop) break;
     }
   }
   __syncthreads();
