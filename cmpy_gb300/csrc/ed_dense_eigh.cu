@@ -31,6 +31,7 @@
 #include <cooperative_groups.h>
 
 #include "ed_common.cuh"
+#include "ed_plan.cuh"
 #include "ed_tridiag.cuh"
 
 namespace ed {
@@ -39,16 +40,45 @@ namespace cg = cooperative_groups;
 
 constexpr int DE_NT = 256;
 
+// Strided batches have a common leading dimension and stride per matrix and per vector; in packed
+// ones (vo, mo: offsets) matrix b takes n_b^2 values at mo[b] and its vectors n_b values at vo[b], so that
+// sectors of very different orders go into one launch without padding.
 struct DenseBatch {
   double* A;          // [B] matrices, row-major
-  int64_t lda, sa;    // leading dimension, matrix stride
+  int64_t lda_, sa;   // strided: leading dimension, matrix stride
   const int* n;       // [B] orders
-  double* d;          // [B][nmax] diagonal of T
-  double* bet;        // [B][nmax] bet[i] couples i-1 and i (bet[0] = 0)
-  double* tau;        // [B][nmax] reflector scales
-  double* P;          // [B][nmax] p, then w
+  double* d;          // diagonal of T
+  double* bet;        // bet[i] couples i-1 and i (bet[0] = 0)
+  double* tau;        // reflector scales
+  double* P;          // p, then w
   double* glim;       // [B][2] Gershgorin bounds of T
-  int nmax;
+  int nmax;           // largest order
+  int vs;             // strided: vector stride
+  const int64_t* vo;  // packed: vector offsets, ascending (else null)
+  const int64_t* mo;  // packed: matrix offsets
+  __device__ __forceinline__ double* mat(int b) const { return A + (vo ? mo[b] : (int64_t)b * sa); }
+  __device__ __forceinline__ int64_t lda(int b) const { return vo ? (int64_t)n[b] : lda_; }
+  __device__ __forceinline__ size_t vec(int b) const { return (size_t)(vo ? vo[b] : (int64_t)b * vs); }
+  // the eigenvectors' matrix (strides ldz, sz when not packed)
+  __device__ __forceinline__ double* zmat(double* Z, int b, int64_t sz) const { return Z + (vo ? mo[b] : (int64_t)b * sz); }
+  __device__ __forceinline__ int64_t zld(int b, int64_t ldz) const { return vo ? (int64_t)n[b] : ldz; }
+  // the e-th vector entry of the B matrices: entry i of matrix b (b = B beyond the last)
+  __device__ __forceinline__ void locate(int64_t e, int B, int* b, int* i) const {
+    if (!vo) {
+      *b = (int)min(e / vs, (int64_t)B);
+      *i = (int)(e - (int64_t)*b * vs);
+      return;
+    }
+    e += vo[0];
+    int lo = 0, hi = B;  // vo[lo] <= e
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (vo[mid] <= e) lo = mid;
+      else hi = mid;
+    }
+    *i = (int)(e - vo[lo]);
+    *b = *i < n[lo] ? lo : B;
+  }
 };
 
 __device__ __forceinline__ double warp_sum_d(double v) {
@@ -62,8 +92,9 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 __global__ void __launch_bounds__(DE_NT) k_hh_column(DenseBatch m, int k) {
   __shared__ double sm[DE_NT / 32];
   const int b = blockIdx.x, n = m.n[b];
+  const int64_t lda = m.lda(b);
   if (k > n - 3) return;
-  double* row = m.A + (size_t)b * m.sa + (size_t)k * m.lda;
+  double* row = m.mat(b) + (size_t)k * lda;
   double s = 0.0;
   for (int i = k + 2 + threadIdx.x; i < n; i += DE_NT) s = fma(row[i], row[i], s);
   s = block_sum<DE_NT>(s, sm);
@@ -77,26 +108,27 @@ __global__ void __launch_bounds__(DE_NT) k_hh_column(DenseBatch m, int k) {
       t = 2.0 / fma(v0, v0, s);
       row[k + 1] = v0;
     }
-    m.tau[(size_t)b * m.nmax + k] = t;
-    m.d[(size_t)b * m.nmax + k] = row[k];
-    m.bet[(size_t)b * m.nmax + k + 1] = alpha;
+    m.tau[m.vec(b) + k] = t;
+    m.d[m.vec(b) + k] = row[k];
+    m.bet[m.vec(b) + k + 1] = alpha;
   }
 }
 
 // step k: p_i = tau sum_{j>k} A[i][j] v_j for i > k (one warp per row)
 __global__ void __launch_bounds__(DE_NT) k_hh_matvec(DenseBatch m, int k) {
   const int b = blockIdx.y, n = m.n[b];
+  const int64_t lda = m.lda(b);
   if (k > n - 3) return;
   const int i = k + 1 + blockIdx.x * (DE_NT / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= n) return;
-  const double t = m.tau[(size_t)b * m.nmax + k];
-  const double* Ab = m.A + (size_t)b * m.sa;
-  const double* v = Ab + (size_t)k * m.lda;
-  const double* ai = Ab + (size_t)i * m.lda;
+  const double t = m.tau[m.vec(b) + k];
+  const double* Ab = m.mat(b);
+  const double* v = Ab + (size_t)k * lda;
+  const double* ai = Ab + (size_t)i * lda;
   double s = 0.0;
   for (int j = k + 1 + lane; j < n; j += 32) s = fma(ai[j], v[j], s);
   s = warp_sum_d(s);
-  if (lane == 0) m.P[(size_t)b * m.nmax + i] = t * s;
+  if (lane == 0) m.P[m.vec(b) + i] = t * s;
 }
 
 // step k, one CTA per matrix: w = p - (tau/2)(p.v) v in place of p
@@ -104,13 +136,14 @@ __global__ void __launch_bounds__(DE_NT) k_hh_dot(DenseBatch m, int k) {
   __shared__ double sm[DE_NT / 32];
   __shared__ double kk;
   const int b = blockIdx.x, n = m.n[b];
+  const int64_t lda = m.lda(b);
   if (k > n - 3) return;
-  const double* v = m.A + (size_t)b * m.sa + (size_t)k * m.lda;
-  double* p = m.P + (size_t)b * m.nmax;
+  const double* v = m.mat(b) + (size_t)k * lda;
+  double* p = m.P + m.vec(b);
   double s = 0.0;
   for (int i = k + 1 + threadIdx.x; i < n; i += DE_NT) s = fma(p[i], v[i], s);
   s = block_sum<DE_NT>(s, sm);
-  if (threadIdx.x == 0) kk = 0.5 * m.tau[(size_t)b * m.nmax + k] * s;
+  if (threadIdx.x == 0) kk = 0.5 * m.tau[m.vec(b) + k] * s;
   __syncthreads();
   for (int i = k + 1 + threadIdx.x; i < n; i += DE_NT) p[i] = fma(-kk, v[i], p[i]);
 }
@@ -118,15 +151,16 @@ __global__ void __launch_bounds__(DE_NT) k_hh_dot(DenseBatch m, int k) {
 // step k: A[i][j] -= v_i w_j + w_i v_j for i, j > k (products rounded separately: symmetric)
 __global__ void __launch_bounds__(DE_NT) k_hh_update(DenseBatch m, int k) {
   const int b = blockIdx.y, n = m.n[b];
+  const int64_t lda = m.lda(b);
   if (k > n - 3) return;
   const int i = k + 1 + blockIdx.x;
   if (i >= n) return;
-  if (m.tau[(size_t)b * m.nmax + k] == 0.0) return;
-  double* Ab = m.A + (size_t)b * m.sa;
-  const double* v = Ab + (size_t)k * m.lda;
-  const double* w = m.P + (size_t)b * m.nmax;
+  if (m.tau[m.vec(b) + k] == 0.0) return;
+  double* Ab = m.mat(b);
+  const double* v = Ab + (size_t)k * lda;
+  const double* w = m.P + m.vec(b);
   const double vi = v[i], wi = w[i];
-  double* ai = Ab + (size_t)i * m.lda;
+  double* ai = Ab + (size_t)i * lda;
   for (int j = k + 1 + threadIdx.x; j < n; j += DE_NT)
     ai[j] = __dsub_rn(ai[j], __dadd_rn(__dmul_rn(vi, w[j]), __dmul_rn(wi, v[j])));
 }
@@ -149,16 +183,17 @@ __global__ void __launch_bounds__(DE_NT) k_hh_cluster(DenseBatch m) {
   __shared__ double kk_s;
   cg::cluster_group cl = cg::this_cluster();
   const int b = blockIdx.y, n = m.n[b];
+  const int64_t lda = m.lda(b);
   double* ps = hsm;           // p, written by every CTA of the cluster
   double* ws = hsm + m.nmax;  // w
   const int rank = (int)cl.block_rank();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gw = rank * (DE_NT / 32) + warp, NW = CS * (DE_NT / 32);
-  double* Ab = m.A + (size_t)b * m.sa;
-  double* tau = m.tau + (size_t)b * m.nmax;
+  double* Ab = m.mat(b);
+  double* tau = m.tau + m.vec(b);
   // reflector of row k (warp 0 of rank 0), as k_hh_column
   auto reflector = [&](int k) {
-    double* row = Ab + (size_t)k * m.lda;
+    double* row = Ab + (size_t)k * lda;
     double sq = 0.0;
     for (int i = k + 2 + lane; i < n; i += 32) sq = fma(row[i], row[i], sq);
     sq = warp_sum_d(sq);
@@ -173,8 +208,8 @@ __global__ void __launch_bounds__(DE_NT) k_hh_cluster(DenseBatch m) {
         row[k + 1] = v0;
       }
       tau[k] = t;
-      m.d[(size_t)b * m.nmax + k] = row[k];
-      m.bet[(size_t)b * m.nmax + k + 1] = alpha;
+      m.d[m.vec(b) + k] = row[k];
+      m.bet[m.vec(b) + k + 1] = alpha;
     }
     __syncwarp();
   };
@@ -182,10 +217,10 @@ __global__ void __launch_bounds__(DE_NT) k_hh_cluster(DenseBatch m) {
   cl.sync();
   for (int k = 0; k + 3 <= n; ++k) {
     const double t = tau[k];
-    const double* v = Ab + (size_t)k * m.lda;
+    const double* v = Ab + (size_t)k * lda;
     // p_i = t sum_{j>k} A[i][j] v_j, one warp per row, into every CTA's copy of p
     for (int i = k + 1 + gw; i < n; i += NW) {
-      const double* ai = Ab + (size_t)i * m.lda;
+      const double* ai = Ab + (size_t)i * lda;
       double sp = 0.0;
       for (int j = k + 1 + lane; j < n; j += 32) sp = fma(ai[j], v[j], sp);
       sp = warp_sum_d(sp);
@@ -204,7 +239,7 @@ __global__ void __launch_bounds__(DE_NT) k_hh_cluster(DenseBatch m) {
     // A[i][j] -= v_i w_j + w_i v_j for i, j > k (products rounded separately: symmetric)
     for (int i = k + 1 + gw; i < n; i += NW) {
       if (t != 0.0) {
-        double* ai = Ab + (size_t)i * m.lda;
+        double* ai = Ab + (size_t)i * lda;
         const double vi = v[i], wi = ws[i];
         for (int j = k + 1 + lane; j < n; j += 32)
           ai[j] = __dsub_rn(ai[j], __dadd_rn(__dmul_rn(vi, ws[j]), __dmul_rn(wi, v[j])));
@@ -229,11 +264,12 @@ __global__ void __launch_bounds__(DE_NTS) k_hh_small(DenseBatch m) {
   __shared__ double sm[DE_NTS / 32];
   __shared__ double sh_t, sh_k;
   const int b = blockIdx.x, n = m.n[b];
+  const int64_t lda = m.lda(b);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double* Ab = m.A + (size_t)b * m.sa;
-  double* p = m.P + (size_t)b * m.nmax;
+  double* Ab = m.mat(b);
+  double* p = m.P + m.vec(b);
   for (int k = 0; k + 3 <= n; ++k) {
-    double* v = Ab + (size_t)k * m.lda;
+    double* v = Ab + (size_t)k * lda;
     // reflector of row k
     double s = 0.0;
     for (int i = k + 2 + tid; i < n; i += DE_NTS) s = fma(v[i], v[i], s);
@@ -248,9 +284,9 @@ __global__ void __launch_bounds__(DE_NTS) k_hh_small(DenseBatch m) {
         t = 2.0 / fma(v0, v0, s);
         v[k + 1] = v0;
       }
-      m.tau[(size_t)b * m.nmax + k] = t;
-      m.d[(size_t)b * m.nmax + k] = v[k];
-      m.bet[(size_t)b * m.nmax + k + 1] = alpha;
+      m.tau[m.vec(b) + k] = t;
+      m.d[m.vec(b) + k] = v[k];
+      m.bet[m.vec(b) + k + 1] = alpha;
       sh_t = t;
     }
     __syncthreads();
@@ -258,7 +294,7 @@ __global__ void __launch_bounds__(DE_NTS) k_hh_small(DenseBatch m) {
     if (t == 0.0) continue;  // uniform: nothing to transform at this step
     // p = tau A22 v, one warp per row
     for (int i = k + 1 + warp; i < n; i += DE_NTS / 32) {
-      const double* ai = Ab + (size_t)i * m.lda;
+      const double* ai = Ab + (size_t)i * lda;
       double acc = 0.0;
       for (int j = k + 1 + lane; j < n; j += 32) acc = fma(ai[j], v[j], acc);
       acc = warp_sum_d(acc);
@@ -278,7 +314,7 @@ __global__ void __launch_bounds__(DE_NTS) k_hh_small(DenseBatch m) {
     const int r = n - k - 1;
     for (int e = tid; e < r * r; e += DE_NTS) {
       const int i = k + 1 + e / r, j = k + 1 + e % r;
-      double* aij = Ab + (size_t)i * m.lda + j;
+      double* aij = Ab + (size_t)i * lda + j;
       *aij = __dsub_rn(*aij, __dadd_rn(__dmul_rn(v[i], p[j]), __dmul_rn(p[i], v[j])));
     }
     __syncthreads();
@@ -293,20 +329,21 @@ __global__ void __launch_bounds__(128) k_hh_finish(DenseBatch m, int B) {
   const int b = blockIdx.x;
   if (b >= B) return;
   const int n = m.n[b];
-  const double* Ab = m.A + (size_t)b * m.sa;
-  double* d = m.d + (size_t)b * m.nmax;
-  double* bt = m.bet + (size_t)b * m.nmax;
+  const int64_t lda = m.lda(b);
+  const double* Ab = m.mat(b);
+  double* d = m.d + m.vec(b);
+  double* bt = m.bet + m.vec(b);
   if (threadIdx.x == 0) {
     bt[0] = 0.0;
     if (n >= 2) {
-      d[n - 2] = Ab[(size_t)(n - 2) * m.lda + n - 2];
-      bt[n - 1] = Ab[(size_t)(n - 2) * m.lda + n - 1];
+      d[n - 2] = Ab[(size_t)(n - 2) * lda + n - 2];
+      bt[n - 1] = Ab[(size_t)(n - 2) * lda + n - 1];
     }
-    d[n - 1] = Ab[(size_t)(n - 1) * m.lda + n - 1];
+    d[n - 1] = Ab[(size_t)(n - 1) * lda + n - 1];
   }
   __syncthreads();
   double lo = d[0], hi = d[0];
-  double* bb = m.P + (size_t)b * m.nmax;
+  double* bb = m.P + m.vec(b);
   for (int i = threadIdx.x; i < n; i += 128) {
     const double r = (i > 0 ? fabs(bt[i]) : 0.0) + (i + 1 < n ? fabs(bt[i + 1]) : 0.0);
     lo = fmin(lo, d[i] - r);
@@ -364,12 +401,13 @@ __global__ void k_tri_eigvals_ms(DenseBatch m, int B, double* W, int P) {
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int gpw = 32 / P, grp = lane / P, j = lane - grp * P;
   const int64_t e = gw * gpw + grp;  // eigenvalue slot over the batch (b, i)
-  const int b = (int)(e / m.nmax), i = (int)(e % m.nmax);
+  int b, i;
+  m.locate(e, B, &b, &i);
   const int n = b < B ? m.n[b] : 0;
   bool done = !(b < B && i < n);  // uniform within a group
-  const double* d = m.d + (size_t)(done ? 0 : b) * m.nmax;
-  const double* bt = m.bet + (size_t)(done ? 0 : b) * m.nmax;
-  const double* bb = m.P + (size_t)(done ? 0 : b) * m.nmax;
+  const double* d = m.d + m.vec(done ? 0 : b);
+  const double* bt = m.bet + m.vec(done ? 0 : b);
+  const double* bb = m.P + m.vec(done ? 0 : b);
   double lo = done ? 0.0 : m.glim[2 * b], hi = done ? 0.0 : m.glim[2 * b + 1];
   const unsigned gmask = (P == 32) ? 0xffffffffu : (((1u << P) - 1u) << (grp * P));
   const double den = 1.0 / (double)(P + 1);
@@ -387,7 +425,7 @@ __global__ void k_tri_eigvals_ms(DenseBatch m, int B, double* W, int P) {
       hi = nhi;
     }
   }
-  if (b < B && i < n && j == 0) W[(size_t)b * m.nmax + i] = 0.5 * (lo + hi);
+  if (b < B && i < n && j == 0) W[m.vec(b) + i] = 0.5 * (lo + hi);
 }
 
 // bytes of shared memory k_tri_eigvecs_warp takes for order n
@@ -403,18 +441,20 @@ __global__ void __launch_bounds__(32) k_tri_eigvecs_warp(DenseBatch m, int B, co
   extern __shared__ __align__(16) double ws[];
   const int lane = threadIdx.x;
   const int64_t e = blockIdx.x;
-  const int b = (int)(e / m.nmax), i0 = (int)(e % m.nmax);
+  int b, i0;
+  m.locate(e, B, &b, &i0);
   if (b >= B) return;
   const int n = m.n[b];
   if (i0 >= n) return;
-  const double* w = W + (size_t)b * m.nmax;
+  const double* w = W + m.vec(b);
   const double ctol = 1e-7 * fmax(1.0, fmax(fabs(w[0]), fabs(w[n - 1])));
   if (i0 > 0 && w[i0] - w[i0 - 1] <= ctol) return;  // not the first member of its cluster
   int i1 = i0 + 1;
   while (i1 < n && w[i1] - w[i1 - 1] <= ctol) ++i1;
-  const double* a = m.d + (size_t)b * m.nmax;
-  const double* bt = m.bet + (size_t)b * m.nmax;
-  double* Zb = Z + (size_t)b * sz;
+  const double* a = m.d + m.vec(b);
+  const double* bt = m.bet + m.vec(b);
+  double* Zb = m.zmat(Z, b, sz);
+  ldz = m.zld(b, ldz);
   double* dd = ws;
   double* du = ws + n;
   double* du2 = ws + 2 * n;
@@ -521,19 +561,21 @@ __global__ void __launch_bounds__(32) k_tri_eigvecs_warp(DenseBatch m, int B, co
 __global__ void k_tri_eigvecs(DenseBatch m, int B, const double* W, double* Z, int64_t ldz, int64_t sz,
                               double* work) {
   const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int b = (int)(g / m.nmax), i0 = (int)(g % m.nmax);
+  int b, i0;
+  m.locate(g, B, &b, &i0);
   if (b >= B) return;
   const int n = m.n[b];
   if (i0 >= n) return;
-  const double* w = W + (size_t)b * m.nmax;
+  const double* w = W + m.vec(b);
   const double ctol = 1e-7 * fmax(1.0, fmax(fabs(w[0]), fabs(w[n - 1])));
   if (i0 > 0 && w[i0] - w[i0 - 1] <= ctol) return;  // not the first member of its cluster
   int i1 = i0 + 1;
   while (i1 < n && w[i1] - w[i1 - 1] <= ctol) ++i1;
-  const double* a = m.d + (size_t)b * m.nmax;
-  const double* bt = m.bet + (size_t)b * m.nmax;
-  double* Zb = Z + (size_t)b * sz;
-  double* wk = work + ((size_t)b * m.nmax + i0) * 5 * (size_t)m.nmax;
+  const double* a = m.d + m.vec(b);
+  const double* bt = m.bet + m.vec(b);
+  double* Zb = m.zmat(Z, b, sz);
+  ldz = m.zld(b, ldz);
+  double* wk = work + (size_t)g * 5 * (size_t)m.nmax;
   double* dd = wk;
   double* du = wk + n;
   double* du2 = wk + 2 * n;
@@ -619,16 +661,18 @@ __global__ void k_tri_eigvecs(DenseBatch m, int B, const double* W, double* Z, i
 __global__ void __launch_bounds__(DE_NT) k_hh_back(DenseBatch m, int B, double* Z, int64_t ldz, int64_t sz) {
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  const int b = (int)(gw / m.nmax), i = (int)(gw % m.nmax);
+  int b, i;
+  m.locate(gw, B, &b, &i);
   if (b >= B) return;
   const int n = m.n[b];
   if (i >= n) return;
-  const double* Ab = m.A + (size_t)b * m.sa;
-  double* y = Z + (size_t)b * sz + (size_t)i * ldz;
+  const int64_t lda = m.lda(b);
+  const double* Ab = m.mat(b);
+  double* y = m.zmat(Z, b, sz) + (size_t)i * m.zld(b, ldz);
   for (int k = n - 3; k >= 0; --k) {
-    const double t = m.tau[(size_t)b * m.nmax + k];
+    const double t = m.tau[m.vec(b) + k];
     if (t == 0.0) continue;
-    const double* v = Ab + (size_t)k * m.lda;
+    const double* v = Ab + (size_t)k * lda;
     double s = 0.0;
     for (int j = k + 1 + lane; j < n; j += 32) s = fma(v[j], y[j], s);
     s = t * warp_sum_d(s);
@@ -689,17 +733,11 @@ static int eigvals_lanes(int64_t E, int sms) {
   return P;
 }
 
-// eigenvalues (ascending) and eigenvectors of the B tridiagonals of m (d, bet, glim and the
-// squared couplings in P set) into W [B][nmax] and Z (row i = eigenvector i). The eigenvectors
-// take the shared-memory kernel when its arrays fit in one CTA's shared memory, else the
-// kernel with global work arrays (5 nmax^2 doubles per matrix, allocated here).
-static ed_status tridiag_eigenpairs(const DeviceContext* ctx, DenseBatch m, int B, double* W, double* Z, int64_t ldz,
-                                    int64_t sz, cudaStream_t s) {
-  const int64_t E = (int64_t)B * m.nmax;
-  const int P = eigvals_lanes(E, ctx->num_sms);
-  const int64_t warps = (E + (32 / P) - 1) / (32 / P);
-  k_tri_eigvals_ms<<<(int)((warps + 3) / 4), 128, 0, s>>>(m, B, W, P);
-  ED_CHECK_LAUNCH("k_tri_eigvals_ms");
+// eigenvectors of the B tridiagonals of m (E entries of vectors), row i of Z = eigenvector i: the
+// shared-memory kernel when its arrays fit in one CTA's shared memory, else the kernel with
+// global work arrays (5 nmax values per eigenvector, allocated here)
+static ed_status tridiag_vectors(const DeviceContext* ctx, DenseBatch m, int B, int64_t E, const double* W, double* Z,
+                                 int64_t ldz, int64_t sz, cudaStream_t s) {
   const size_t sm = eigvec_smem(m.nmax);
   if (sm + 1024 <= (size_t)ctx->smem_optin) {
     static std::atomic<uint64_t> done{0};
@@ -721,6 +759,93 @@ static ed_status tridiag_eigenpairs(const DeviceContext* ctx, DenseBatch m, int 
   ED_CUDA(cudaFreeAsync(work, s));
   if (e != cudaSuccess) return cuda_fail(e, "k_tri_eigvecs");
   return ED_OK;
+}
+
+// all eigenvalues (ascending) of the B tridiagonals of m (d, bet, glim and the squared couplings in P set)
+static ed_status tridiag_values(const DeviceContext* ctx, DenseBatch m, int B, int64_t E, double* W, cudaStream_t s) {
+  const int P = eigvals_lanes(E, ctx->num_sms);
+  const int64_t warps = (E + (32 / P) - 1) / (32 / P);
+  k_tri_eigvals_ms<<<(int)((warps + 3) / 4), 128, 0, s>>>(m, B, W, P);
+  ED_CHECK_LAUNCH("k_tri_eigvals_ms");
+  return ED_OK;
+}
+
+// A = Q T Q^T of the batch, in the form that suits its largest order
+static ed_status householder(const DeviceContext* ctx, DenseBatch m, int B, cudaStream_t s) {
+  if (m.nmax <= DE_SMALL) {  // every step of each matrix in one CTA
+    k_hh_small<<<B, DE_NTS, 0, s>>>(m);
+    ED_CHECK_LAUNCH("Householder (one CTA per matrix)");
+    return ED_OK;
+  }
+  // orders above DE_SMALL: one cluster of 16 (else 8) CTAs per matrix while the clusters'
+  // SMs do the FP64 work faster than per-step launches over every SM would (order <= 640, or a
+  // batch that occupies the GPU with clusters); else four launches per step
+  // CMPY_ED_HH_CLUSTER=16, 8 or 0 forces that cluster size or the per-step launches (for tests
+  // and comparisons; read once per process)
+  static int env_cluster = -2;
+  if (env_cluster == -2) {
+    const char* e = getenv("CMPY_ED_HH_CLUSTER");
+    env_cluster = e ? atoi(e) : -1;
+  }
+  const bool want = env_cluster >= 0 ? env_cluster > 0
+                                     : (m.nmax <= DE_CLUSTER_MAX || (int64_t)B * 16 >= ctx->num_sms);
+  if (want) {
+    ed_status st = ED_OK;
+    if (env_cluster != 8 && hh_cluster_launch<16>(ctx, m, B, s, &st)) return st;
+    if (hh_cluster_launch<8>(ctx, m, B, s, &st)) return st;
+  }
+  const int rows_per = DE_NT / 32;
+  for (int k = 0; k + 3 <= m.nmax; ++k) {
+    const int rem = m.nmax - k - 1;
+    k_hh_column<<<B, DE_NT, 0, s>>>(m, k);
+    k_hh_matvec<<<dim3((rem + rows_per - 1) / rows_per, B), DE_NT, 0, s>>>(m, k);
+    k_hh_dot<<<B, DE_NT, 0, s>>>(m, k);
+    k_hh_update<<<dim3(rem, B), DE_NT, 0, s>>>(m, k);
+    ED_CHECK_LAUNCH_N("Householder step", 4);
+  }
+  return ED_OK;
+}
+
+static ed_status back_transform(DenseBatch m, int B, int64_t E, double* Z, int64_t ldz, int64_t sz, cudaStream_t s) {
+  k_hh_back<<<(int)((E * 32 + DE_NT - 1) / DE_NT), DE_NT, 0, s>>>(m, B, Z, ldz, sz);
+  ED_CHECK_LAUNCH("k_hh_back");
+  return ED_OK;
+}
+
+// a packed batch (host arrays, orders non-increasing): the orders fall into at most three ranges (one
+// CTA, one cluster or per-step launches per matrix) whose reductions and eigenvectors are launched apart;
+// eigenvalues and the back-transformation take the whole batch
+static ed_status eigh_packed(const DeviceContext* ctx, DenseBatch m, const int* n, const int64_t* vo, int B, double* W,
+                             double* Z, cudaStream_t s) {
+  const int64_t E = vo[B];
+  auto part = [&](int b0, int* count, int64_t* e) {  // the batch from matrix b0 on, and its range
+    DenseBatch r = m;
+    r.n += b0;
+    r.vo += b0;
+    r.mo += b0;
+    r.glim += 2 * b0;
+    r.nmax = n[b0];
+    auto kind = [&](int k) { return n[k] <= DE_SMALL ? 0 : (n[k] <= DE_CLUSTER_MAX ? 1 : 2); };
+    int b1 = b0 + 1;
+    while (b1 < B && kind(b1) == kind(b0)) ++b1;
+    *count = b1 - b0;
+    *e = vo[b1] - vo[b0];
+    return r;
+  };
+  int c = 0;
+  int64_t e = 0;
+  for (int b = 0; b < B; b += c) {
+    const DenseBatch r = part(b, &c, &e);
+    ED_TRY(householder(ctx, r, c, s));
+  }
+  k_hh_finish<<<B, 128, 0, s>>>(m, B);
+  ED_CHECK_LAUNCH("k_hh_finish");
+  ED_TRY(tridiag_values(ctx, m, B, E, W, s));
+  for (int b = 0; b < B; b += c) {
+    const DenseBatch r = part(b, &c, &e);
+    ED_TRY(tridiag_vectors(ctx, r, c, e, W, Z, 0, 0, s));
+  }
+  return back_transform(m, B, E, Z, 0, 0, s);
 }
 
 }  // namespace ed
@@ -747,9 +872,9 @@ ED_API ed_status ed_dense_eigh_batch(double* d_a, int64_t lda, int64_t stride_a,
   ED_CUDA(cudaMallocAsync((void**)&buf, (4 * nm + 2 * (size_t)B) * sizeof(double), s));
   ED_CUDA(cudaMallocAsync((void**)&dn, (size_t)B * sizeof(int), s));
   ED_CUDA(cudaMemcpyAsync(dn, h_n, (size_t)B * sizeof(int), cudaMemcpyHostToDevice, s));
-  DenseBatch m;
+  DenseBatch m{};
   m.A = d_a;
-  m.lda = lda;
+  m.lda_ = lda;
   m.sa = stride_a;
   m.n = dn;
   m.d = buf;
@@ -758,58 +883,68 @@ ED_API ed_status ed_dense_eigh_batch(double* d_a, int64_t lda, int64_t stride_a,
   m.P = buf + 3 * nm;
   m.glim = buf + 4 * nm;
   m.nmax = n_max;
-  ed_status st = ED_OK;
-  const int rows_per = DE_NT / 32;
-  if (n_max <= DE_SMALL) {
-    // every step of each matrix in one CTA
-    k_hh_small<<<B, DE_NTS, 0, s>>>(m);
-    const cudaError_t e = cudaGetLastError();
-    count_launches(1);
-    if (e != cudaSuccess) st = cuda_fail(e, "Householder (one CTA per matrix)");
-  }
-  // orders above DE_SMALL: one cluster of 16 (else 8) CTAs per matrix while the clusters'
-  // SMs do the FP64 work faster than per-step launches over every SM would (order <= 640, or a
-  // batch that occupies the GPU with clusters); else four launches per step
-  // CMPY_ED_HH_CLUSTER=16, 8 or 0 forces that cluster size or the per-step launches (for tests
-  // and comparisons; read once per process)
-  static int env_cluster = -2;
-  if (env_cluster == -2) {
-    const char* e = getenv("CMPY_ED_HH_CLUSTER");
-    env_cluster = e ? atoi(e) : -1;
-  }
-  bool stepped = n_max <= DE_SMALL;
-  const bool want = env_cluster >= 0 ? env_cluster > 0
-                                     : (n_max <= DE_CLUSTER_MAX || (int64_t)B * 16 >= ctx->num_sms);
-  if (!stepped && want) {
-    if (env_cluster != 8) stepped = hh_cluster_launch<16>(ctx, m, B, s, &st);
-    if (!stepped) stepped = hh_cluster_launch<8>(ctx, m, B, s, &st);
-  }
-  for (int k = 0; !stepped && k + 3 <= n_max && st == ED_OK; ++k) {
-    const int rem = n_max - k - 1;
-    k_hh_column<<<B, DE_NT, 0, s>>>(m, k);
-    k_hh_matvec<<<dim3((rem + rows_per - 1) / rows_per, B), DE_NT, 0, s>>>(m, k);
-    k_hh_dot<<<B, DE_NT, 0, s>>>(m, k);
-    k_hh_update<<<dim3(rem, B), DE_NT, 0, s>>>(m, k);
-    const cudaError_t e = cudaGetLastError();
-    count_launches(4);
-    if (e != cudaSuccess) st = cuda_fail(e, "Householder step");
-  }
+  m.vs = n_max;
+  ed_status st = householder(ctx, m, B, s);
   if (st == ED_OK) {
     k_hh_finish<<<B, 128, 0, s>>>(m, B);
     const cudaError_t e = cudaGetLastError();
     count_launches(1);
     if (e != cudaSuccess) st = cuda_fail(e, "k_hh_finish");
   }
-  if (st == ED_OK) st = tridiag_eigenpairs(ctx, m, B, d_w, d_z, ldz, stride_z, s);
-  if (st == ED_OK) {
-    const int64_t nt = (int64_t)B * n_max;
-    k_hh_back<<<(int)((nt * 32 + DE_NT - 1) / DE_NT), DE_NT, 0, s>>>(m, B, d_z, ldz, stride_z);
-    const cudaError_t e = cudaGetLastError();
-    count_launches(1);
-    if (e != cudaSuccess) st = cuda_fail(e, "k_hh_back");
-  }
+  if (st == ED_OK) st = tridiag_values(ctx, m, B, (int64_t)nm, d_w, s);
+  if (st == ED_OK) st = tridiag_vectors(ctx, m, B, (int64_t)nm, d_w, d_z, ldz, stride_z, s);
+  if (st == ED_OK) st = back_transform(m, B, (int64_t)nm, d_z, ldz, stride_z, s);
   cudaFreeAsync(buf, s);
   cudaFreeAsync(dn, s);
+  return st;
+}
+
+ED_API ed_status ed_sector_eigh(const ed_plan* plans, int B, double* d_w, double* d_z, ed_stream_t stream) {
+  if (B < 1 || !plans || !d_w || !d_z) return fail(ED_ERR_INVALID_ARG, "null pointer or B < 1");
+  std::vector<int64_t> off(2 * (size_t)B + 2);
+  std::vector<int> n(B);
+  int64_t* vo = off.data();
+  int64_t* mo = off.data() + B + 1;
+  for (int b = 0; b < B; ++b) {
+    ED_TRY(check_plan(plans[b]));
+    const int64_t d = plans[b]->dim;
+    if (d < 1) return fail(ED_ERR_INVALID_ARG, "empty sector");
+    if (d > 32768) return fail(ED_ERR_TOO_LARGE, "ed_sector_eigh: dimension above 32768");
+    n[b] = (int)d;
+    if (b > 0 && n[b] > n[b - 1]) return fail(ED_ERR_INVALID_ARG, "sectors must come in descending order of size");
+    vo[b + 1] = vo[b] + d;
+    mo[b + 1] = mo[b] + d * d;
+  }
+  DeviceContext* ctx;
+  ED_TRY(device_context(&ctx));
+  cudaStream_t s = as_stream(stream);
+  // the matrices, d, bet, tau, P, Gershgorin bounds, the offsets and the orders in one allocation
+  const size_t nm = (size_t)vo[B], na = (size_t)mo[B], nd = na + 4 * nm + 2 * (size_t)B;
+  const size_t head = off.size() * sizeof(int64_t) + ((size_t)B * sizeof(int) + 7) / 8 * 8;
+  char* buf = nullptr;
+  ED_CUDA(cudaMallocAsync((void**)&buf, head + nd * sizeof(double), s));
+  int64_t* d_off = (int64_t*)buf;
+  int* d_n = (int*)(d_off + off.size());
+  DenseBatch m{};
+  m.A = (double*)(buf + head);
+  m.n = d_n;
+  m.d = m.A + na;
+  m.bet = m.d + nm;
+  m.tau = m.bet + nm;
+  m.P = m.tau + nm;
+  m.glim = m.P + nm;
+  m.nmax = n[0];
+  m.vo = d_off;
+  m.mo = d_off + B + 1;
+  auto run = [&]() -> ed_status {
+    ED_CUDA(cudaMemcpyAsync(d_off, off.data(), off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s));
+    ED_CUDA(cudaMemcpyAsync(d_n, n.data(), (size_t)B * sizeof(int), cudaMemcpyHostToDevice, s));
+    ED_CUDA(cudaMemsetAsync(m.A, 0, na * sizeof(double), s));
+    for (int b = 0; b < B; ++b) ED_TRY(dense_into(plans[b], m.A + mo[b], s));
+    return eigh_packed(ctx, m, n.data(), vo, B, d_w, d_z, s);
+  };
+  const ed_status st = run();
+  cudaFreeAsync(buf, s);
   return st;
 }
 
@@ -834,11 +969,13 @@ ED_API ed_status ed_tridiag_eigh(const double* d_alpha, const double* d_beta, in
   b.P = buf + 3 * (size_t)m;
   b.glim = buf + 4 * (size_t)m;
   b.nmax = m;
+  b.vs = m;
   k_tri_setup<<<1, 1, 0, s>>>(b, d_alpha, d_beta, m);
   const cudaError_t e = cudaGetLastError();
   count_launches(1);
   ed_status st = e != cudaSuccess ? cuda_fail(e, "k_tri_setup") : ED_OK;
-  if (st == ED_OK) st = tridiag_eigenpairs(ctx, b, 1, d_w, d_z, ldz, (int64_t)m * ldz, s);
+  if (st == ED_OK) st = tridiag_values(ctx, b, 1, m, d_w, s);
+  if (st == ED_OK) st = tridiag_vectors(ctx, b, 1, m, d_w, d_z, ldz, (int64_t)m * ldz, s);
   cudaFreeAsync(buf, s);
   cudaFreeAsync(dn, s);
   return st;

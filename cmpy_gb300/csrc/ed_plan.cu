@@ -467,6 +467,17 @@ __global__ void k_spin_dense(SpinArgs a, double* __restrict__ out, int64_t D) {
   }
 }
 
+ed_status dense_into(const ed_plan_s* p, double* out, cudaStream_t s) {
+  if (p->kind == 0) {
+    k_hub_dense<<<grid_for(p->dim, 128, 4096), 128, 0, s>>>(hub_args(p), p->fp, out, p->dim);
+  } else {
+    SpinArgs a{p->spin_diag, p->up.off, p->up.idx, p->up.coef, p->dim};
+    k_spin_dense<<<grid_for(p->dim, 128, 4096), 128, 0, s>>>(a, out, p->dim);
+  }
+  ED_CHECK_LAUNCH("ed_dense");
+  return ED_OK;
+}
+
 }  // namespace ed
 
 using namespace ed;
@@ -672,14 +683,7 @@ ED_API ed_status ed_dense(ed_plan p, double* out, ed_stream_t stream) {
   if (!out) return fail(ED_ERR_INVALID_ARG, "null output");
   cudaStream_t s = as_stream(stream);
   ED_CUDA(cudaMemsetAsync(out, 0, (size_t)p->dim * p->dim * sizeof(double), s));
-  if (p->kind == 0) {
-    k_hub_dense<<<grid_for(p->dim, 128, 4096), 128, 0, s>>>(hub_args(p), p->fp, out, p->dim);
-  } else {
-    SpinArgs a{p->spin_diag, p->up.off, p->up.idx, p->up.coef, p->dim};
-    k_spin_dense<<<grid_for(p->dim, 128, 4096), 128, 0, s>>>(a, out, p->dim);
-  }
-  ED_CHECK_LAUNCH("ed_dense");
-  return ED_OK;
+  return dense_into(p, out, s);
 }
 
 ED_API ed_status ed_diagonal(ed_plan p, double* out, ed_stream_t stream) {

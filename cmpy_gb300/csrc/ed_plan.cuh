@@ -228,6 +228,8 @@ ed_status check_plan(const ed_plan_s* p);
 // y = H x for nvec vectors (leading dimension ld); skipped when *stop != 0 (stop may be null).
 ed_status matvec_f64(const ed_plan_s* p, const double* x, double* y, int64_t nvec, int64_t ld, cudaStream_t s,
                      const int* stop = nullptr);
+// H as a dense row-major matrix into zeroed memory
+ed_status dense_into(const ed_plan_s* p, double* out, cudaStream_t s);
 // Builds p->bfp when the sector qualifies (called at plan creation); its tables go into `arena`.
 bool bfp_possible(const ed_plan_s* p);
 ed_status build_bfp(ed_plan_s* p, const HostTable& hu, const HostTable& hd, DeviceArena& arena);

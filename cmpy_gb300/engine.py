@@ -565,6 +565,28 @@ def dense_eigh(a: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     return dense_eigh_batch([a])[0]
 
 
+def sector_eigh(plans, chunk_bytes: int = 1 << 30):
+    """Every eigenpair of the sectors' Hamiltonians, many sectors to a launch: yields lists of
+    (index into plans, eigenvalues ascending [n], eigenvectors as columns [n, n]), largest sectors
+    first, each list of at most ``chunk_bytes`` of eigenvectors (or one sector)."""
+    plans = list(plans)
+    order = sorted(range(len(plans)), key=lambda i: -plans[i].dim)
+    while order:
+        size, take = 0, 0
+        while take < len(order) and (take == 0 or size + 8 * plans[order[take]].dim ** 2 <= chunk_bytes):
+            size += 8 * plans[order[take]].dim ** 2
+            take += 1
+        idx, order = order[:take], order[take:]
+        dims = [plans[i].dim for i in idx]
+        with plans[idx[0]]._dev():
+            W = torch.empty(sum(dims), dtype=torch.float64, device=device())
+            Z = torch.zeros(sum(d * d for d in dims), dtype=torch.float64, device=device())
+            h = (C.c_void_p * take)(*[plans[i].handle for i in idx])
+            N.check(N.lib().ed_sector_eigh(h, take, N.ptr(W), N.ptr(Z), _stream()))
+        ws, zs = W.split(dims), Z.split([d * d for d in dims])
+        yield [(i, w, z.view(d, d).t()) for i, d, w, z in zip(idx, dims, ws, zs)]
+
+
 def tridiag_eigh(alpha: torch.Tensor, beta: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     """Every eigenpair of the tridiagonal (alpha[0..m), beta[1..m)): (eigenvalues ascending,
     eigenvectors as columns [m, m]) on the device."""

@@ -317,6 +317,12 @@ ED_API ed_status ed_tridiag_pinv_solve_batch(const double* d_alpha, int lda, con
 ED_API ed_status ed_dense_eigh_batch(double* d_a, int64_t lda, int64_t stride_a, const int* h_n, int B, int n_max,
                                      double* d_w, double* d_z, int64_t ldz, int64_t stride_z,
                                      ed_stream_t stream);
+/* Every eigenpair of the Hamiltonians of B sectors in the same launches (solve_sector of every
+ * sector, cmpy/exactdiag.py:46-57, 215-245). The plans come in descending order of dimension;
+ * sector b's eigenvalues (ascending) and eigenvectors (row i of a contiguous n_b x n_b matrix) follow
+ * those of sector b - 1 in d_w (sum n_b) and d_z (sum n_b^2). Asynchronous on `stream` (work
+ * memory from cudaMallocAsync: sum n_b^2 + 4 sum n_b doubles). */
+ED_API ed_status ed_sector_eigh(const ed_plan* plans, int B, double* d_w, double* d_z, ed_stream_t stream);
 /* Every eigenpair of the symmetric tridiagonal (d_alpha[0..m), d_beta[1..m)): eigenvalues
  * ascending -> d_w, eigenvector i -> row i of d_z (leading dimension ldz). The same bisection
  * and inverse iteration as ed_dense_eigh_batch; used for the real-time Green's function of a
