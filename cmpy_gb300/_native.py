@@ -181,6 +181,8 @@ _SIGNATURES = {
     "ed_batch_tape_reverse": (I32, [PLAN, I32, P, P, C.POINTER(C.c_int), I32, I32, P, P, P, P, P, P, P, P,
                                     C.c_size_t, P, P, P]),
     "ed_plan_fixed_point": (I32, [PLAN]),
+    "ed_plan_resident": (I32, [PLAN]),
+    "ed_random_start": (I32, [P, I64, C.c_uint64, P]),
     "ed_fixed_from_f64": (I32, [P, I64, I32, P, C.POINTER(C.c_int32), P]),
     "ed_fixed_to_f64": (I32, [P, I64, C.c_int32, P, P]),
     "ed_matvec_fixed": (I32, [PLAN, P, C.c_int32, P, C.POINTER(C.c_int32), C.POINTER(I32), P]),

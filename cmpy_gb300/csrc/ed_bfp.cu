@@ -2433,6 +2433,8 @@ ED_API ed_status ed_plan_set_matvec_variant(ed_plan p, int variant) {
   return ED_OK;
 }
 
+ED_API int ed_plan_resident(ed_plan p) { return p && resident_fits(p) ? 1 : 0; }
+
 ED_API int ed_plan_fixed_point(ed_plan p) { return (p && p->bfp.eligible) ? p->bfp.m_in : 0; }
 
 }  // extern "C"

@@ -387,6 +387,17 @@ static ed_status use_fixed(const ed_plan_s* p, const ed_lanczos_params* prm, boo
   return ED_OK;
 }
 
+ED_API ed_status ed_random_start(double* d_v, int64_t n, uint64_t seed, ed_stream_t stream) {
+  if (n < 0) return fail(ED_ERR_INVALID_ARG, "negative n");
+  if (n == 0) return ED_OK;
+  if (!d_v) return fail(ED_ERR_INVALID_ARG, "null vector");
+  DeviceContext* ctx;
+  ED_TRY(device_context(&ctx));
+  k_random_start<<<grid_for(n, 256, ctx->num_sms * 8), 256, 0, as_stream(stream)>>>(d_v, n, seed);
+  ED_CHECK_LAUNCH("k_random_start");
+  return ED_OK;
+}
+
 ED_API ed_status ed_lanczos_workspace(ed_plan p, const ed_lanczos_params* prm, size_t* bytes) {
   ED_TRY(check_plan(p));
   if (!prm || !bytes) return fail(ED_ERR_INVALID_ARG, "null argument");

@@ -227,6 +227,11 @@ class Plan:
         return int(N.lib().ed_plan_fixed_point(self._h))
 
     @property
+    def resident(self) -> bool:
+        """A Lanczos run of the sector is one launch (its vectors fit a cluster's shared memory)."""
+        return bool(N.lib().ed_plan_resident(self._h))
+
+    @property
     def matvec_variant(self) -> int:
         """Fixed-point matvec the plan uses: 7 = single-pass kernel with the dn states renumbered
         by hop count (default where it fits), 3/2/1 = single-pass kernels in the sector's order,
@@ -446,6 +451,13 @@ def lanczos(plan: Plan, max_steps: int = 250, reorth: bool = False, want_vector:
         m = int(res.steps)
         return LanczosResult(float(res.energy), float(res.residual), m, int(res.converged), alpha[:m],
                              beta[: m + 1], vec, float(res.matvec_ms), int(res.matvecs))
+
+
+def random_start(n: int, seed: int = 0) -> torch.Tensor:
+    """The seeded uniform (0, 1) start vector of a Lanczos run (a prefix of every longer one)."""
+    out = torch.empty(n, dtype=torch.float64, device=device())
+    N.check(N.lib().ed_random_start(N.ptr(out), int(n), int(seed), _stream()))
+    return out
 
 
 def lanczos_coeffs(plan: Plan, start: torch.Tensor, max_steps: int = 200,

@@ -249,6 +249,8 @@ typedef struct ed_lanczos_result {
   int32_t matvecs;       /* matvec launches timed */
 } ed_lanczos_result;
 
+/* The uniform (0, 1) start vector that a Lanczos run without one generates from its seed. */
+ED_API ed_status ed_random_start(double* d_v, int64_t n, uint64_t seed, ed_stream_t stream);
 /* Bytes of caller-provided device workspace for ed_lanczos (Krylov basis included). */
 ED_API ed_status ed_lanczos_workspace(ed_plan plan, const ed_lanczos_params* params,
                                       size_t* h_bytes);
@@ -487,6 +489,9 @@ ED_API ed_status ed_cf_adjoint(const double* d_alpha, const double* d_beta, int 
  * ed_plan_fixed_point: m_in > 0 (the input mantissa bound 2^m_in) when the sector has a
  * fixed-point matvec (one hopping magnitude, eps/U/t exact integers times 2^-F), else 0. */
 ED_API int ed_plan_fixed_point(ed_plan plan);
+/* 1 when a fixed-point Lanczos run of the sector is one launch of a thread-block cluster (its vectors fit
+ * the cluster's shared memory and no matvec variant or wait limit was asked for), else 0. */
+ED_API int ed_plan_resident(ed_plan plan);
 /* d_xm = round(d_x * 2^-e) with max |d_xm| < 2^m_bits; *h_exp = e. Synchronous. */
 ED_API ed_status ed_fixed_from_f64(const double* d_x, int64_t n, int m_bits, int64_t* d_xm,
                                    int32_t* h_exp, ed_stream_t stream);
