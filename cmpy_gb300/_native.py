@@ -182,6 +182,7 @@ _SIGNATURES = {
                                     C.c_size_t, P, P, P]),
     "ed_plan_fixed_point": (I32, [PLAN]),
     "ed_plan_resident": (I32, [PLAN]),
+    "ed_spectrum_bounds": (I32, [PLAN, P, P]),
     "ed_random_start": (I32, [P, I64, C.c_uint64, P]),
     "ed_fixed_from_f64": (I32, [P, I64, I32, P, C.POINTER(C.c_int32), P]),
     "ed_fixed_to_f64": (I32, [P, I64, C.c_int32, P, P]),

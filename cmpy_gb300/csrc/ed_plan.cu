@@ -316,6 +316,7 @@ static ed_status finish_bounds(ed_plan_s* p, cudaStream_t s) {
   memcpy(&h0, &hm[0], 8);
   memcpy(&h1, &hm[1], 8);
   p->hnorm_bound = diag_max + h0 + h1;
+  p->hop_bound = h0 + h1;
   ED_CUDA(cudaStreamSynchronize(s));
   return ED_OK;
 }
@@ -543,6 +544,7 @@ ED_API ed_status ed_plan_create_fermion(const ed_fermion_model* m, int n_up, int
       host_bounds(hd, &rd, &edn);
       for (double v : p->u) su += std::fabs(v);
       p->hnorm_bound = (eu + edn + su) + ru + rd;
+      p->hop_bound = ru + rd;
       const TableOffsets o = place_table(p->up, hu, arena);
       if (same) share_table(p->dn, o, arena);
       else place_table(p->dn, hd, arena);
@@ -684,6 +686,36 @@ ED_API ed_status ed_dense(ed_plan p, double* out, ed_stream_t stream) {
   cudaStream_t s = as_stream(stream);
   ED_CUDA(cudaMemsetAsync(out, 0, (size_t)p->dim * p->dim * sizeof(double), s));
   return dense_into(p, out, s);
+}
+
+// Gershgorin: the extremes of the diagonal (the lowest and highest site energies filled, as many double
+// occupations as the fillings force or allow), widened by the largest row of hoppings
+ED_API ed_status ed_spectrum_bounds(ed_plan p, double* lo, double* hi) {
+  ED_TRY(check_plan(p));
+  if (!lo || !hi) return fail(ED_ERR_INVALID_ARG, "null output");
+  if (p->kind != 0) {
+    *lo = -p->hnorm_bound;
+    *hi = p->hnorm_bound;
+    return ED_OK;
+  }
+  std::vector<double> e = p->eps, u = p->u;
+  std::sort(e.begin(), e.end());
+  std::sort(u.begin(), u.end());
+  const int n = p->n_sites, k0 = std::max(0, p->n_up + p->n_dn - n), k1 = std::min(p->n_up, p->n_dn);
+  double a = 0.0, b = 0.0;
+  for (int s = 0; s < 2; ++s)
+    for (int i = 0; i < (s ? p->n_dn : p->n_up); ++i) {
+      a += e[i];
+      b += e[n - 1 - i];
+    }
+  for (int i = 0; i < k1; ++i) {
+    if (i < k0 || u[i] < 0.0) a += u[i];
+    if (i < k0 || u[n - 1 - i] > 0.0) b += u[n - 1 - i];
+  }
+  const double pad = p->hop_bound + 1e-12 * p->hnorm_bound;
+  *lo = a - pad;
+  *hi = b + pad;
+  return ED_OK;
 }
 
 ED_API ed_status ed_diagonal(ed_plan p, double* out, ed_stream_t stream) {

@@ -199,6 +199,7 @@ struct ed_plan_s {
   int64_t num_up = 0, num_dn = 0, dim = 0;
   int64_t nnz = 0;
   double hnorm_bound = 0.0;
+  double hop_bound = 0.0;  // largest row sum of |hopping|
   // model copy (host)
   std::vector<double> eps, u;
   std::vector<int32_t> b1, b2;

@@ -226,6 +226,12 @@ class Plan:
         """Input mantissa bits of the sector's integer matvec, 0 if it has none."""
         return int(N.lib().ed_plan_fixed_point(self._h))
 
+    def spectrum_bounds(self) -> tuple[float, float]:
+        """An interval that holds every eigenvalue of the sector."""
+        lo, hi = C.c_double(), C.c_double()
+        N.check(N.lib().ed_spectrum_bounds(self._h, C.byref(lo), C.byref(hi)))
+        return float(lo.value), float(hi.value)
+
     @property
     def resident(self) -> bool:
         """A Lanczos run of the sector is one launch (its vectors fit a cluster's shared memory)."""

@@ -160,6 +160,8 @@ ED_API ed_status ed_matmat(ed_plan plan, const double* d_x, double* d_y, int64_t
 /* Dense H (row-major D x D) for small sectors, summed in triplet order like
  * HamiltonOperator.toarray (cmpy/operators.py:632-635). D <= 32768. */
 ED_API ed_status ed_dense(ed_plan plan, double* d_out, ed_stream_t stream);
+/* An interval that holds every eigenvalue of the sector (host call). */
+ED_API ed_status ed_spectrum_bounds(ed_plan plan, double* h_lo, double* h_hi);
 /* Diagonal of H (HamiltonOperator._trace sums it, cmpy/operators.py:641-646). */
 ED_API ed_status ed_diagonal(ed_plan plan, double* d_out, ed_stream_t stream);
 
