@@ -191,6 +191,7 @@ _SIGNATURES = {
     "ed_plan_set_wait_limit": (I32, [PLAN, I64]),
     "ed_plan_set_matvec_variant": (I32, [PLAN, I32]),
     "ed_gf_continued_fraction": (I32, [P, P, I32, F64, F64, I32, P, I64, P, I32, P]),
+    "ed_thermal_sums": (I32, [P, I64, P, I64, I64, P, I64, I64, I32, I32, I32, F64, F64, P, P]),
     "ed_lehmann_accumulate": (I32, [P, I64, P, I64, P, F64, F64, P, I64, P, P]),
     "ed_tevo_sum": (I32, [P, P, I64, F64, I32, P, I64, P, I32, P]),
     "ed_tevo_krylov": (I32, [P, P, I32, F64, F64, I32, P, I64, F64, P, I32, C.POINTER(I32), P]),

@@ -52,13 +52,15 @@ def _stream():
     return N.stream_handle()
 
 
-def _as_dev_f64(x) -> torch.Tensor:
+def _strided_dev_f64(x) -> torch.Tensor:
     dev = device()
     if isinstance(x, torch.Tensor):
-        t = x.to(device=dev, dtype=torch.float64)
-    else:
-        t = torch.as_tensor(np.asarray(x, dtype=np.float64)).to(dev)
-    return t.contiguous()
+        return x.to(device=dev, dtype=torch.float64)
+    return torch.as_tensor(np.asarray(x, dtype=np.float64)).to(dev)
+
+
+def _as_dev_f64(x) -> torch.Tensor:
+    return _strided_dev_f64(x).contiguous()
 
 
 def _as_dev_states(states) -> torch.Tensor:
@@ -294,7 +296,7 @@ class Plan:
         """c^dag (create) or c on site pos, spin sigma (1 up, 2 dn), into the target sector.
         x: (D,) or (D, k)."""
         with self._dev():
-            x = _as_dev_f64(x)
+            x = _strided_dev_f64(x)
             vec = x.ndim == 1
             X = x.reshape(self.dim, -1).t().contiguous()
             k = X.shape[0]
@@ -710,6 +712,22 @@ def laplace_t2z(times, gf_t, z, method: str = "lin") -> torch.Tensor:
                                    N.ptr(torch.view_as_real(zt)), zt.numel(), m, N.ptr(torch.view_as_real(out)),
                                    _stream()))
     return out
+
+
+def thermal_sums(evals, evecs, up_states, dn_states, site: int, dn: bool, beta: float, emin: float,
+                 occ: bool = True) -> tuple[float, float, float, float]:
+    """(smallest energy E, sum_k w_k, sum_k w_k <n_site>_k, sum_k w_k <n_up n_dn>_k) over a sector's
+    eigenpairs (vectors as columns), w_k = exp(-beta (E_k - min(emin, E)))."""
+    e = _as_dev_f64(evals).reshape(-1)
+    v = _strided_dev_f64(evecs)
+    nu, nd = len(up_states), len(dn_states)
+    if v.ndim != 2 or v.shape != (nu * nd, e.numel()):
+        raise ValueError("eigenvectors must be (states, eigenvalues)")
+    st = _as_dev_states(np.concatenate([np.asarray(up_states, np.int64), np.asarray(dn_states, np.int64)])) if occ else None
+    out = (C.c_double * 4)()
+    N.check(N.lib().ed_thermal_sums(N.ptr(e), e.numel(), N.ptr(v), v.stride(0), v.stride(1), N.ptr(st), nu, nd, int(site),
+                                    int(bool(dn)), int(bool(occ)), float(beta), float(emin), out, _stream()))
+    return tuple(out)
 
 
 def lehmann_accumulate(evals, evals_p1, overlap, beta: float, emin: float, z, g: torch.Tensor) -> torch.Tensor:

@@ -140,7 +140,7 @@ def _solve_sector_dev(model, sector: Sector, cache: dict = None):
     key = (sector.n_up, sector.n_dn)
     if cache is not None and key in cache:
         w, v = cache[key]
-        return E._as_dev_f64(w), E._as_dev_f64(v)
+        return E._as_dev_f64(w), E._strided_dev_f64(v)
     w, v = _dense_eigh(_sector_plan(model, sector.n_up, sector.n_dn))
     if cache is not None:
         cache[key] = [w, v]
@@ -219,8 +219,8 @@ def double_occupation(up_states, dn_states, evals, evecs, beta, emin, pos):
 def accumulate_gf(gf, z, cdag, evals, evecs, evals_p1, evecs_p1, beta, emin=0.0):
     """gf += Lehmann poles of one sector pair (cmpy/exactdiag.py:110-134). `cdag` is a
     CreationOperator (its device map is used); `gf` is a complex128 torch CUDA tensor."""
-    V = E._as_dev_f64(evecs)
-    Vp = E._as_dev_f64(evecs_p1)
+    V = E._strided_dev_f64(evecs)  # (the solver's eigenvectors are rows in memory, as the map takes them)
+    Vp = E._strided_dev_f64(evecs_p1)
     CV = cdag._apply_dev(V)
     ov = (Vp.t() @ CV) ** 2
     return E.lehmann_accumulate(evals, evals_p1, ov, float(beta), float(emin), z, gf)
@@ -265,21 +265,21 @@ class GreensFunctionMeasurement:
 
     def accumulate(self, sector, sector_p1, evals, evecs, evals_p1, evecs_p1, cdag):
         evals_t = E._as_dev_f64(evals)
-        min_energy = float(evals_t.min().item())
+        up, dn = sector.up_states, sector.dn_states
+        min_energy, part, occ, double = E.thermal_sums(evals_t, evecs, up, dn, self.pos, self.sigma != UP, self.beta,
+                                                       self._gs_energy, self._measure_occ)
         factor = 1.0
         if min_energy < self._gs_energy:
             factor = float(np.exp(-self.beta * (self._gs_energy - min_energy)))
             self._gs_energy = min_energy
         e0 = self._gs_energy
-        self._part = self._part * factor + float(torch.exp(-self.beta * (evals_t - e0)).sum().item())
+        self._part = self._part * factor + part
         if factor != 1.0:
             self._gf *= factor
         accumulate_gf(self._gf, self._zt, cdag, evals_t, evecs, evals_p1, evecs_p1, self.beta, e0)
         if self._measure_occ:
-            up, dn = sector.up_states, sector.dn_states
-            self._occ = self._occ * factor + occupation(up, dn, evals_t, evecs, self.beta, e0, self.pos, self.sigma)
-            self._occ_double = self._occ_double * factor + double_occupation(up, dn, evals_t, evecs, self.beta, e0,
-                                                                             self.pos)
+            self._occ = self._occ * factor + occ
+            self._occ_double = self._occ_double * factor + double
 
 
 def gf_lehmann(model, z, beta, pos=0, sigma=UP, eig_cache=None, occ=True, jw_sign: bool = False):
@@ -321,8 +321,8 @@ def _lehmann_pair(model, z, beta, i, j, sigma, eig_cache, jw_sign):
         part = part * factor + float(torch.exp(-beta * (w_t - e0)).sum().item())
         if factor != 1.0:
             gf *= factor
-        V = E._as_dev_f64(v)
-        Vp = E._as_dev_f64(vp)
+        V = E._strided_dev_f64(v)
+        Vp = E._strided_dev_f64(vp)
         a_i = Vp.t() @ CreationOperator(sector, sector_p1, pos=i, sigma=sigma, jw_sign=jw_sign)._apply_dev(V)
         if j == i:
             ov = a_i**2

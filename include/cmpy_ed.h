@@ -552,6 +552,15 @@ ED_API ed_status ed_gf_continued_fraction(const double* d_alpha, const double* d
                                           const double* d_z, int64_t n_z, double* d_g,
                                           int accumulate, ed_stream_t stream);
 
+/* Thermal sums of one sector (cmpy/exactdiag.py:60-107, 137-212): h_out = {E = the smallest eigenvalue,
+ * Z = sum_k w_k, sum_k w_k <n_site>_k, sum_k w_k <n_up n_dn>_k}, w_k = exp(-beta (E_k - min(emin, E))).
+ * Element i = u * n_dn_states + d of eigenvector k at d_evecs[i * row_stride + k * col_stride]; d_states:
+ * the up, then the dn states (bits = sites); dn: the species of <n_site>; occ = 0 leaves the last two
+ * zero. Waits for `stream`. */
+ED_API ed_status ed_thermal_sums(const double* d_evals, int64_t n, const double* d_evecs, int64_t row_stride,
+                                 int64_t col_stride, const int64_t* d_states, int64_t n_up_states,
+                                 int64_t n_dn_states, int site, int dn, int occ, double beta, double emin,
+                                 double* h_out, ed_stream_t stream);
 /* Lehmann pole sum of cmpy/exactdiag.py:110-129 (_accumulate_sum): with the overlap
  * matrix ov[m, n] = |<m|c^dag|n>|^2 (FP64, d_p1 x d, row-major), adds
  *   sum_{m,n} ov[m,n] (w_n + w'_m) / (z - E'_m + E_n),  w = exp(-beta (E - emin))
