@@ -52,7 +52,7 @@ struct TapeState {
   unsigned int ticket[4];
 };
 
-__device__ __forceinline__ bool tp_stopped(const int* stop) { return stop && *(volatile const int*)stop != 0; }
+__device__ __forceinline__ bool tp_stopped(const int* stop) { return stop && block_flag(stop); }
 
 // *res = <a, b> (and sqrt -> *res_sqrt)
 __global__ void __launch_bounds__(TP_NT) k_tp_dot(const double* __restrict__ a, const double* __restrict__ b,

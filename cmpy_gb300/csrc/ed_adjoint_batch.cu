@@ -79,6 +79,10 @@ __device__ __forceinline__ bool bskip(const int* gate, int mode, int k, int b) {
   if (mode == 2) return k >= gate[b];
   return false;
 }
+// the same for all threads of a block (mode 1 gates are set by convergence tests on another stream)
+__device__ __forceinline__ bool bt_skip(const int* gate, int mode, int k, int b) {
+  return mode == 1 ? block_flag(&gate[b]) : bskip(gate, mode, k, b);
+}
 
 // y[b] = H_b x[b] for BMV_PB problems per CTA: one CTA per (up-row, group of problems), threads
 // over the dn index. The hop lists are loaded once for the group and each problem keeps its
@@ -153,7 +157,7 @@ __global__ void __launch_bounds__(BT_NT) k_bt_dot(const double* __restrict__ a, 
                                                   double* partial, unsigned int* ticket, double* res, int64_t rstride,
                                                   double* rsq, int64_t qstride, const int* gate, int mode, int k) {
   const int b = blockIdx.y, G = gridDim.x;
-  if (bskip(gate, mode, k, b)) return;
+  if (bt_skip(gate, mode, k, b)) return;
   __shared__ double sm[BT_NT / 32];
   const double* ab = a + (int64_t)b * n;
   const double* cb = c + (int64_t)b * n;
@@ -175,7 +179,7 @@ __global__ void __launch_bounds__(BT_NT) k_bt_dot(const double* __restrict__ a, 
 __global__ void k_bt_scale(const double* __restrict__ v, double* __restrict__ out, int64_t n, const double* scale,
                            int64_t sstride, const int* gate, int mode, int k) {
   const int b = blockIdx.y;
-  if (bskip(gate, mode, k, b)) return;
+  if (bt_skip(gate, mode, k, b)) return;
   const double s = 1.0 / scale[b * sstride];
   const double* vb = v + (int64_t)b * n;
   double* ob = out + (int64_t)b * n;
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(BT_NT) k_bt_update(double* __restrict__ w, con
                                                      double* beta, int K, int k, double breakdown, double* partial,
                                                      BState bs) {
   const int b = blockIdx.y, G = gridDim.x;
-  if (bs.stop[b]) return;
+  if (block_flag(&bs.stop[b])) return;
   __shared__ double sm[BT_NT / 32];
   const double a = alpha[(int64_t)b * K + k], bk = qp ? beta[(int64_t)b * (K + 1) + k] : 0.0;
   double* wb = w + (int64_t)b * n;

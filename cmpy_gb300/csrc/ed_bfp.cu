@@ -238,7 +238,7 @@ template <int NT, bool VEC2, bool DIAG64>
 __global__ void __launch_bounds__(NT) k_bfp_hub_matvec(BfpHubArgs a, const int64_t* __restrict__ X,
                                                       int64_t* __restrict__ W, double* partial,
                                                       unsigned long long* partial_max, BfpState* st) {
-  if (st && *(volatile int*)&st->stop) return;
+  if (st && block_flag(&st->stop)) return;
   extern __shared__ int64_t xs[];  // [2*nd + 1]
   __shared__ double smd[NT / 32];
   __shared__ unsigned long long smu[NT / 32];
@@ -345,7 +345,7 @@ template <bool DIAG64>
 __global__ void __launch_bounds__(MV2_NT, 1) k_bfp_hub_matvec2(BfpHubArgs a, const int64_t* __restrict__ X,
                                                               int64_t* __restrict__ W, double* partial,
                                                               unsigned long long* partial_max, BfpState* st) {
-  if (st && *(volatile int*)&st->stop) return;
+  if (st && block_flag(&st->stop)) return;
   extern __shared__ int64_t smem[];
   __shared__ double smd[MV2_NT / 32];
   __shared__ unsigned long long smu[MV2_NT / 32];
@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(MV3_MAXNT, 1)
                       const int32_t* __restrict__ up_lst, const int32_t* __restrict__ up_cnt,
                       const int64_t* __restrict__ X, int64_t* W, double* partial,
                       unsigned long long* partial_max, BfpState* st, int* status, BfpFuse fz, long wait_limit) {
-  if (st && *(volatile int*)&st->stop) return;
+  if (st && block_flag(&st->stop)) return;
   extern __shared__ __align__(128) unsigned char sm3[];
   __shared__ double smd[MV3_MAXNT / 32];
   __shared__ unsigned long long smu[MV3_MAXNT / 32];
@@ -866,7 +866,7 @@ __global__ void __launch_bounds__(UP_NT, 2)
     k_bfp_up_panels(const int32_t* __restrict__ up_off, const int32_t* __restrict__ up_npos,
                     const int32_t* __restrict__ up_idx, int64_t nu, int64_t nd, const int64_t* __restrict__ X,
                     int64_t* __restrict__ W, const BfpState* st) {
-  if (st && *(const volatile int*)&st->stop) return;
+  if (st && block_flag(&st->stop)) return;
   extern __shared__ __align__(16) longlong2 pan[];  // [nu][2]: columns c0..c0+3 of every row
   const int64_t npan = nd / MV_PW;
   for (int64_t pnl = blockIdx.x; pnl < npan; pnl += gridDim.x) {
@@ -918,7 +918,7 @@ __global__ void __launch_bounds__(UP_NT, 2)
 __global__ void k_bfp_scalars(BfpVecs v, int k, int F, int m_in, const double* partial,
                               const unsigned long long* partial_max, int nparts, double* alpha, const double* beta,
                               BfpState* st) {
-  if (*(volatile int*)&st->stop) return;
+  if (block_flag(&st->stop)) return;
   __shared__ double sm[BT / 32];
   __shared__ unsigned long long smu[BT / 32];
   double t = 0.0;
@@ -997,7 +997,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(BT, 4) k_bfp_update(BfpVecs v, int k, const int64_t* __restrict__ W, double* partial,
                                                    unsigned long long* partial_max, double* beta,
                                                    const double* alpha, BfpState* st, int final_k) {
-  if (*(volatile int*)&st->stop) return;
+  if (block_flag(&st->stop)) return;
   __shared__ double sm[BT / 32];
   __shared__ unsigned long long smu[BT / 32];
   const int64_t Aw = st->A_w, Aq = st->A_q, Ap = k > 0 ? st->A_p : 0;

@@ -129,6 +129,14 @@ __device__ __forceinline__ double rcp_f64(double x) {
   return fma(y, fma(e, e, e), y);
 }
 
+// Whether the block returns early: the same answer for all its threads. A run's stop flag is set from
+// another stream while the step kernels run (ed_lzcheck.cuh), so threads of one block that read it for
+// themselves can disagree, and those that go on would then meet shared memory and barriers that
+// the others never set up.
+__device__ __forceinline__ bool block_flag(const int* flag) {
+  return __syncthreads_or(*(const volatile int*)flag) != 0;
+}
+
 // ---- deterministic block reduction -------------------------------------------------------
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double* smem /*[NT/32]*/) {

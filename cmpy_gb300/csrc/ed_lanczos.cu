@@ -31,7 +31,7 @@ struct LzState {
   unsigned int ticket[8];
 };
 
-__device__ __forceinline__ bool lz_stopped(const LzState* st) { return *(volatile const int*)&st->stop != 0; }
+__device__ __forceinline__ bool lz_stopped(const LzState* st) { return block_flag(&st->stop); }
 __device__ __forceinline__ bool lz_skip(const LzState* st, int pass) {
   return lz_stopped(st) || (pass == 1 && *(volatile const int*)&st->settled != 0);
 }
@@ -72,7 +72,7 @@ __global__ void k_random_start(double* v, int64_t n, uint64_t seed) {
 // out = <a, b> (or ||a||^2 with b == a); result -> *res (and optionally its sqrt -> *res_sqrt)
 __global__ void k_dot(const double* __restrict__ a, const double* __restrict__ b, int64_t n, double* partial,
                       LzState* st, int tk, double* res, double* res_sqrt, const int* stop) {
-  if (stop && *(volatile const int*)stop) return;
+  if (stop && block_flag(stop)) return;
   __shared__ double sm[LZ_NT / 32];
   double v = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)LZ_NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * LZ_NT)

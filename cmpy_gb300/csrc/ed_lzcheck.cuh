@@ -46,7 +46,7 @@ __device__ __forceinline__ void tri_hint(const TriResult* tr, double* lo, double
 static __global__ void __launch_bounds__(TRI_NT) k_tri_check(const double* alpha, const double* beta, int m, double tol,
                                                             int* stop, int* steps, TriResult* tr, double* cvec,
                                                             double* work) {
-  if (*(volatile int*)stop) return;  // converged, invariant subspace or failed wait already
+  if (block_flag(stop)) return;  // converged, invariant subspace or failed wait already
   double lo, hi;
   tri_hint(tr, &lo, &hi);
   const double e = tridiag_lowest_block<TRI_SM>(alpha, beta, m, cvec, work, lo, hi);
@@ -65,7 +65,7 @@ static __global__ void __launch_bounds__(TRI_NT) k_tri_check_batch(const double*
                                                                   int m, double tol, int* stop, int* steps,
                                                                   double* cvec, double* work, int ldw) {
   const int b = blockIdx.x;
-  if (*(volatile int*)&stop[b]) return;
+  if (block_flag(&stop[b])) return;
   const double* a = alpha + (size_t)b * lda;
   const double* bb = beta + (size_t)b * (lda + 1);
   double* c = cvec + (size_t)b * ldw;

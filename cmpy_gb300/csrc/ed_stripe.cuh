@@ -92,7 +92,7 @@ __host__ __device__ constexpr size_t stripe_smem(int64_t n) { return (size_t)(n 
 // ---- pass 1: S = A X, 4-column stripes ---------------------------------------------------------
 __global__ void __launch_bounds__(ST_NT, 2)
     k_stripe_up(StripeArgs a, const int64_t* __restrict__ X, int64_t* __restrict__ S, BfpState* st) {
-  if (st && *(volatile int*)&st->stop) return;
+  if (st && block_flag(&st->stop)) return;
   extern __shared__ __align__(128) unsigned char sm_stu[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t nu = a.nu, nd = a.nd;
@@ -156,7 +156,7 @@ template <bool DIAG64>
 __global__ void __launch_bounds__(ST_NT, 2)
     k_stripe_dn(BfpHubArgs h, StripeArgs a, StripeDiag dg, const int64_t* __restrict__ X, int64_t* W,
                 double* partial, unsigned long long* partial_max, BfpState* st, BfpFuse fz) {
-  if (st && *(volatile int*)&st->stop) return;
+  if (st && block_flag(&st->stop)) return;
   extern __shared__ __align__(128) unsigned char sm_std[];
   __shared__ double smd[ST_NT / 32];
   __shared__ unsigned long long smu[ST_NT / 32];

@@ -125,7 +125,7 @@ __device__ __forceinline__ void sweep_drain(uint64_t* bar, uint64_t* lbar, int r
 // ---- pass 1: S = A X, column stripes -----------------------------------------------------------
 __global__ void __launch_bounds__(SW_NT, 2)
     k_sweep_up(SweepArgs a, const int64_t* __restrict__ X, int64_t* __restrict__ S, BfpState* st, int* status) {
-  if (st && *(volatile int*)&st->stop) return;
+  if (st && block_flag(&st->stop)) return;
   extern __shared__ __align__(128) unsigned char sm_up[];
   int64_t* ring = (int64_t*)sm_up;                                                 // [ring * SW_CH][SW_W]
   uint16_t* lring = (uint16_t*)(sm_up + (size_t)a.ring * SW_CH * SW_W * 8);       // [SW_LR][SW_CH][SW_LST]
@@ -255,7 +255,7 @@ template <bool DIAG64>
 __global__ void __launch_bounds__(SW_NT, 2)
     k_sweep_dn(BfpHubArgs h, SweepArgs a, SweepDiag dg, const int64_t* __restrict__ X, int64_t* W, double* partial,
                unsigned long long* partial_max, BfpState* st, int* status, BfpFuse fz) {
-  if (st && *(volatile int*)&st->stop) return;
+  if (st && block_flag(&st->stop)) return;
   extern __shared__ __align__(128) unsigned char sm_dn[];
   __shared__ double smd[SW_NT / 32];
   __shared__ unsigned long long smu[SW_NT / 32];
