@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(TP_NT) k_tp_radot(double* __restrict__ qb1, co
                                                     const double* __restrict__ qm, int64_t n, const double* beta,
                                                     double* abar, double* bbar, int k, double* partial,
                                                     unsigned int* ticket, double* res) {
-  __shared__ double sm[TP_NT / 32];
+  __shared__ double rows[5 * TP_NT];
   const int G = gridDim.x;
   const double ce = ext ? ext_coef[k + 1] : 0.0;
   const bool fin = res != nullptr;
@@ -209,14 +209,11 @@ __global__ void __launch_bounds__(TP_NT) k_tp_radot(double* __restrict__ qb1, co
     }
   }
   const int nd = fin ? 1 : 5;
-  double dv[5] = {d1, d2, d3, d4, d5};
-  for (int j = 0; j < nd; ++j) {
-    const double s = block_sum<TP_NT>(dv[j], sm);
-    if (threadIdx.x == 0) partial[(int64_t)j * G + blockIdx.x] = s;
-  }
+  const double dv[5] = {d1, d2, d3, d4, d5};
+  tp_block_rows(dv, nd, rows, partial + blockIdx.x, G);
   if (tp_last_block(ticket)) {
     double t[5];
-    for (int j = 0; j < nd; ++j) t[j] = tp_row_sum(partial + (int64_t)j * G, G, sm);
+    tp_rows_total(partial, G, nd, G, t);
     if (threadIdx.x == 0) {
       if (fin) {
         *res = t[0];
@@ -245,8 +242,9 @@ __global__ void __launch_bounds__(SW_NT) k_tp_rstep(SandwichArgs g, int ns, int 
                                                     const double* alpha, const double* beta, const double* abar,
                                                     const double* bbar, int k, int has_next, int first,
                                                     double* __restrict__ pracc, double* __restrict__ psw) {
-  extern __shared__ double sacc[];  // [P][SW_NT]
-  sandwich_zero(sacc, P);
+  extern __shared__ double sacc[];  // [nb][SW_NT]: the hop parameters
+  const int nb = P - 2 * ns;
+  sandwich_zero(sacc, nb);
   const double ak = alpha[k], ab = abar[k];
   const double inv = has_next ? 1.0 / beta[k + 1] : 0.0, bb1 = has_next ? bbar[k + 1] : 0.0;
   const double bk = k > 0 ? beta[k] : 0.0;
@@ -260,9 +258,9 @@ __global__ void __launch_bounds__(SW_NT) k_tp_rstep(SandwichArgs g, int ns, int 
     wbar[i] = wb;
     // w_bar^T (dH/dtheta) q_k, row i: the hop part now, the diagonal part through sum_k w_bar q_k
     pracc[i] = fma(wb, x0, first ? 0.0 : pracc[i]);
-    sandwich_hop_terms(g, ns, i, wb, q0, sacc + threadIdx.x);
+    sandwich_hop_terms(g, 0, i, wb, q0, sacc + threadIdx.x);
   }
-  sandwich_block_out(sacc, P, psw + (int64_t)blockIdx.x * SW_P, true);
+  sandwich_block_out(sacc, nb, psw + (int64_t)blockIdx.x * SW_P + 2 * ns, true);
 }
 
 // the diagonal (eps, U) part of sum_k w_bar_k^T (dH/dtheta) q_k from pracc = sum_k w_bar_k q_k,
@@ -557,7 +555,7 @@ ED_API ed_status ed_tape_reverse(ed_plan p, int m, int ckpt, const double* d_alp
                                         nullptr);
         ED_CHECK_LAUNCH("k_tp_radot");
       }
-      k_tp_rstep<<<L.nsw, SW_NT, sandwich_smem(P), s>>>(g, p->n_sites, P, has_next ? qb(k + 1) : nullptr, has_next ? q(k + 1) : nullptr, q(k),
+      k_tp_rstep<<<L.nsw, SW_NT, sandwich_smem(P - 2 * p->n_sites), s>>>(g, p->n_sites, P, has_next ? qb(k + 1) : nullptr, has_next ? q(k + 1) : nullptr, q(k),
                                          Ws + (int64_t)(k - s0) * D, qb(k), k > 0 ? qb(k - 1) : nullptr, wbar,
                                          d_alpha, d_beta, AB, BB, k, has_next ? 1 : 0, k == m - 1 ? 1 : 0, pracc,
                                          psw);

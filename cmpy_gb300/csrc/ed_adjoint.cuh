@@ -37,22 +37,23 @@ __device__ __forceinline__ void sandwich_diag_terms(const SandwichArgs& g, int n
   for (uint64_t bits = su & sd; bits; bits &= bits - 1) acc[(ns + __ffsll((long long)bits) - 1) * SW_NT] += pr;
 }
 
-__device__ __forceinline__ void sandwich_hop_terms(const SandwichArgs& g, int ns, int64_t i, double ai,
+// (p0: row of the first hop parameter. At most 16 sites: fewer than 2^31 states, 32-bit division)
+__device__ __forceinline__ void sandwich_hop_terms(const SandwichArgs& g, int p0, int64_t i, double ai,
                                                    const double* __restrict__ b, double* acc) {
-  const int64_t u = i / g.nd, d = i - u * g.nd;
+  const int64_t u = (uint32_t)i / (uint32_t)g.nd, d = i - u * g.nd;
   // the hop's sign (that of its coefficient) flips the sign bit of a_i: integer operations
   const long long ab = __double_as_longlong(ai);
   const long long sbit = (long long)0x8000000000000000ull;
   const int32_t u0 = g.up_off[u], u1 = g.up_off[u + 1];
   for (int32_t e = u0; e < u1; ++e) {
     const double as = __longlong_as_double(ab ^ (__double_as_longlong(g.up_coef[e]) & sbit));
-    double* a = acc + (2 * ns + g.up_bond[e]) * SW_NT;
+    double* a = acc + (p0 + g.up_bond[e]) * SW_NT;
     *a = fma(as, b[(int64_t)g.up_idx[e] * g.nd + d], *a);
   }
   const int32_t d0 = g.dn_off[d], d1 = g.dn_off[d + 1];
   for (int32_t e = d0; e < d1; ++e) {
     const double as = __longlong_as_double(ab ^ (__double_as_longlong(g.dn_coef[e]) & sbit));
-    double* a = acc + (2 * ns + g.dn_bond[e]) * SW_NT;
+    double* a = acc + (p0 + g.dn_bond[e]) * SW_NT;
     *a = fma(as, b[u * g.nd + g.dn_idx[e]], *a);
   }
 }
@@ -60,7 +61,7 @@ __device__ __forceinline__ void sandwich_hop_terms(const SandwichArgs& g, int ns
 __device__ __forceinline__ void sandwich_row(const SandwichArgs& g, int ns, int64_t i, double ai, double bi,
                                              const double* __restrict__ b, double* acc) {
   sandwich_diag_terms(g, ns, i, ai * bi, acc);
-  sandwich_hop_terms(g, ns, i, ai, b, acc);
+  sandwich_hop_terms(g, 2 * ns, i, ai, b, acc);
 }
 
 __device__ __forceinline__ void sandwich_zero(double* sacc, int P) {
@@ -99,6 +100,43 @@ __device__ __forceinline__ double tp_row_sum(const double* partial, int nb, doub
   double v = 0.0;
   for (int b = threadIdx.x; b < nb; b += TP_NT) v += ((volatile const double*)partial)[b];
   return block_sum<TP_NT>(v, sm);
+}
+
+// nr <= NR block sums, row j -> out[j * stride], from one shared-memory transpose: a warp per row. (A
+// shuffle tree per row and warp is 5 NR additions in every warp, each 64 cycles of the FP64 pipe; this is
+// 12 in one warp per row. Reductions were a quarter of k_bt_radot.) rows: NR * TP_NT doubles
+template <int NR>
+__device__ __forceinline__ void tp_block_rows(const double (&v)[NR], int nr, double* rows, double* out,
+                                              int64_t stride) {
+#pragma unroll
+  for (int j = 0; j < NR; ++j)
+    if (j < nr) rows[j * TP_NT + threadIdx.x] = v[j];
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int j = threadIdx.x >> 5; j < nr; j += TP_NT / 32) {
+    const double* r = rows + j * TP_NT + lane;
+    double s = ((r[0] + r[32]) + (r[64] + r[96])) + ((r[128] + r[160]) + (r[192] + r[224]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[j * stride] = s;
+  }
+}
+// the last block's sums of nr rows of nb partials, a warp per row, all valid in every thread afterwards
+template <int NR>
+__device__ __forceinline__ void tp_rows_total(const double* partial, int64_t stride, int nr, int nb, double (&t)[NR]) {
+  __shared__ double tot[NR];
+  const int lane = threadIdx.x & 31;
+  for (int j = threadIdx.x >> 5; j < nr; j += TP_NT / 32) {
+    double s = 0.0;
+    for (int b = lane; b < nb; b += 32) s += ((volatile const double*)partial)[j * stride + b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) tot[j] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < NR; ++j)
+    if (j < nr) t[j] = tot[j];
 }
 
 // the residual of step k, element i (shared by the forward and the recompute)

@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(BT_NT) k_bt_radot(double* __restrict__ qb1, co
   const int b = blockIdx.y, B = gridDim.y, G = gridDim.x;
   const bool fin = res != nullptr;
   if (k + 1 >= bs.m[b]) return;
-  __shared__ double sm[BT_NT / 32];
+  __shared__ double rows[5 * BT_NT];
   const int64_t o = (int64_t)b * n;
   const double ce = ext ? ext_coef[(int64_t)b * K + k + 1] : 0.0;
   double d1 = 0.0, d2 = 0.0, d3 = 0.0, d4 = 0.0, d5 = 0.0;
@@ -331,14 +331,11 @@ __global__ void __launch_bounds__(BT_NT) k_bt_radot(double* __restrict__ qb1, co
     }
   }
   const int nd = fin ? 1 : 5;
-  double dv[5] = {d1, d2, d3, d4, d5};
-  for (int j = 0; j < nd; ++j) {
-    const double s = block_sum<BT_NT>(dv[j], sm);
-    if (threadIdx.x == 0) partial[((int64_t)j * B + b) * G + blockIdx.x] = s;
-  }
+  const double dv[5] = {d1, d2, d3, d4, d5};
+  tp_block_rows(dv, nd, rows, partial + (int64_t)b * G + blockIdx.x, (int64_t)B * G);
   if (tp_last_block(&bs.ticket[b])) {
     double t[5];
-    for (int j = 0; j < nd; ++j) t[j] = bt_row_sum(partial + ((int64_t)j * B + b) * G, G, sm);
+    tp_rows_total(partial + (int64_t)b * G, (int64_t)B * G, nd, G, t);
     if (threadIdx.x == 0) {
       if (fin) {
         res[b] = t[0];
@@ -358,6 +355,10 @@ __global__ void __launch_bounds__(BT_NT) k_bt_radot(double* __restrict__ qb1, co
 
 // reverse step k, part 2, per problem with k < m[b] (the single tape's k_tp_rstep), fused with
 // w_bar^T (dH_b/dtheta) q_k added to the block's row of psw[b][blk][SW_P]
+// (Bound by the FP64 pipe. The accumulators are those of the hop parameters alone: with the 2 ns rows
+// that stay zero here, zeroing and adding them up was a third of the kernel's FP64 instructions and its shared
+// memory kept half of the warps off an SM. With tp_block_rows in k_bt_radot, 64 problems of 63,504
+// states, forward and backward: 308 -> 269 ms.)
 __global__ void __launch_bounds__(SW_NT) k_bt_rstep(SandwichArgs g, int ns, int P, const double* __restrict__ qb1,
                                                     const double* __restrict__ q1, const double* __restrict__ q0,
                                                     const double* __restrict__ w0, double* __restrict__ qbk,
@@ -368,8 +369,9 @@ __global__ void __launch_bounds__(SW_NT) k_bt_rstep(SandwichArgs g, int ns, int 
   const int b = blockIdx.y;
   const int m = bs.m[b];
   if (k >= m) return;
-  extern __shared__ double sacc[];  // [P][SW_NT]
-  sandwich_zero(sacc, P);
+  extern __shared__ double sacc[];  // [nb][SW_NT]: the hop parameters
+  const int nb = P - 2 * ns;
+  sandwich_zero(sacc, nb);
   const bool has_next = k + 1 < m, first = k == m - 1;
   const double ak = alpha[(int64_t)b * K + k], ab = abar[(int64_t)b * K + k];
   const double inv = has_next ? 1.0 / beta[(int64_t)b * (K + 1) + k + 1] : 0.0;
@@ -386,9 +388,9 @@ __global__ void __launch_bounds__(SW_NT) k_bt_rstep(SandwichArgs g, int ns, int 
     wbar[o + i] = wb;
     // the hop part now, the diagonal part through sum_k w_bar_k q_k
     pracc[o + i] = fma(wb, x0, first ? 0.0 : pracc[o + i]);
-    sandwich_hop_terms(g, ns, i, wb, q0b, sacc + threadIdx.x);
+    sandwich_hop_terms(g, 0, i, wb, q0b, sacc + threadIdx.x);
   }
-  sandwich_block_out(sacc, P, psw + ((int64_t)b * gridDim.x + blockIdx.x) * SW_P, true);
+  sandwich_block_out(sacc, nb, psw + ((int64_t)b * gridDim.x + blockIdx.x) * SW_P + 2 * ns, true);
 }
 
 // the diagonal (eps, U) part from pracc[b] = sum_k w_bar_k q_k (problems with m[b] >= 1)
@@ -757,7 +759,7 @@ ED_API ed_status ed_batch_tape_reverse(ed_plan p, int B, const double* d_theta, 
         const double* q1 = q(k + 1) ? q(k + 1) : q(k);
         k_bt_radot<<<gv, BT_NT, 0, s>>>(qb(k + 1), tmp, d_ext_vec, d_ext_coef, q1, q(k), k > 0 ? q(k - 1) : nullptr,
                                         D, d_beta, AB, BB, K, k, part, bs, nullptr);
-        k_bt_rstep<<<gw, SW_NT, sandwich_smem(P), s>>>(g, p->n_sites, P, qb(k + 1), q1, q(k),
+        k_bt_rstep<<<gw, SW_NT, sandwich_smem(P - 2 * p->n_sites), s>>>(g, p->n_sites, P, qb(k + 1), q1, q(k),
                                                       Ws + (int64_t)(k - s0) * BD, qb(k), k > 0 ? qb(k - 1) : nullptr,
                                                       wbar, d_alpha, d_beta, AB, BB, K, k, bs, pracc, psw);
         launch_bmv(p, B, d_theta, d_diag, wbar, tmp, bs.m, 2, k, s);
