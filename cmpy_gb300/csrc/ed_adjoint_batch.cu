@@ -73,10 +73,11 @@ __device__ __forceinline__ double bhop(double sign, double t) {
   return __longlong_as_double(__double_as_longlong(t) ^ (__double_as_longlong(sign) & (long long)0x8000000000000000ull));
 }
 
-// problem b is skipped when mode 1: gate[b] != 0, mode 2: k >= gate[b]
+// problem b is skipped when mode 1: gate[b] != 0, mode 2: k >= gate[b], mode 3: k != gate[b]
 __device__ __forceinline__ bool bskip(const int* gate, int mode, int k, int b) {
   if (mode == 1) return gate[b] != 0;
   if (mode == 2) return k >= gate[b];
+  if (mode == 3) return k != gate[b];
   return false;
 }
 // the same for all threads of a block (mode 1 gates are set by convergence tests on another stream)
@@ -355,16 +356,19 @@ __global__ void __launch_bounds__(BT_NT) k_bt_radot(double* __restrict__ qb1, co
 
 // reverse step k, part 2, per problem with k < m[b] (the single tape's k_tp_rstep), fused with
 // w_bar^T (dH_b/dtheta) q_k added to the block's row of psw[b][blk][SW_P]
+// whole: every q is on the tape, and w_k = H q_k of a step with a successor is what the recurrence made it,
+// beta_{k+1} q_{k+1} + alpha_k q_k + beta_k q_{k-1}: three FP64 operations an element, H takes eleven.
 // (Bound by the FP64 pipe. The accumulators are those of the hop parameters alone: with the 2 ns rows
 // that stay zero here, zeroing and adding them up was a third of the kernel's FP64 instructions and its shared
 // memory kept half of the warps off an SM. With tp_block_rows in k_bt_radot, 64 problems of 63,504
 // states, forward and backward: 308 -> 269 ms.)
 __global__ void __launch_bounds__(SW_NT) k_bt_rstep(SandwichArgs g, int ns, int P, const double* __restrict__ qb1,
                                                     const double* __restrict__ q1, const double* __restrict__ q0,
-                                                    const double* __restrict__ w0, double* __restrict__ qbk,
-                                                    double* __restrict__ qbm, double* __restrict__ wbar,
-                                                    const double* alpha, const double* beta, const double* abar,
-                                                    const double* bbar, int K, int k, BState bs,
+                                                    const double* __restrict__ qm, const double* __restrict__ w0,
+                                                    double* __restrict__ qbk, double* __restrict__ qbm,
+                                                    double* __restrict__ wbar, const double* alpha,
+                                                    const double* beta, const double* abar, const double* bbar, int K,
+                                                    int k, int whole, BState bs,
                                                     double* __restrict__ pracc, double* __restrict__ psw) {
   const int b = blockIdx.y;
   const int m = bs.m[b];
@@ -374,7 +378,8 @@ __global__ void __launch_bounds__(SW_NT) k_bt_rstep(SandwichArgs g, int ns, int 
   sandwich_zero(sacc, nb);
   const bool has_next = k + 1 < m, first = k == m - 1;
   const double ak = alpha[(int64_t)b * K + k], ab = abar[(int64_t)b * K + k];
-  const double inv = has_next ? 1.0 / beta[(int64_t)b * (K + 1) + k + 1] : 0.0;
+  const double b1 = has_next ? beta[(int64_t)b * (K + 1) + k + 1] : 0.0;
+  const double inv = has_next ? 1.0 / b1 : 0.0;
   const double bb1 = has_next ? bbar[(int64_t)b * (K + 1) + k + 1] : 0.0;
   const double bk = k > 0 ? beta[(int64_t)b * (K + 1) + k] : 0.0;
   const int64_t D = g.nu * g.nd, o = (int64_t)b * D;
@@ -383,7 +388,14 @@ __global__ void __launch_bounds__(SW_NT) k_bt_rstep(SandwichArgs g, int ns, int 
     const double rb = has_next ? fma(bb1, q1[o + i], qb1[o + i] * inv) : 0.0;
     const double x0 = q0b[i];
     const double wb = fma(ab, x0, rb);
-    qbk[o + i] = fma(ab, w0[o + i], fma(-ak, rb, first ? 0.0 : qbk[o + i]));
+    double w;
+    if (whole && has_next) {
+      w = fma(b1, q1[o + i], ak * x0);
+      if (qm) w = fma(bk, qm[o + i], w);
+    } else {
+      w = w0[o + i];
+    }
+    qbk[o + i] = fma(ab, w, fma(-ak, rb, first ? 0.0 : qbk[o + i]));
     if (qbm) qbm[o + i] = -bk * rb;
     wbar[o + i] = wb;
     // the hop part now, the diagonal part through sum_k w_bar_k q_k
@@ -468,7 +480,7 @@ size_t bt_align(size_t x) { return (x + 255) & ~(size_t)255; }
 BLayout blayout(const ed_plan_s* p, int B, int K, int c) {
   BLayout L;
   const int64_t D = p->dim;
-  L.nvec = std::max(4, 2 * c + 6);
+  L.nvec = c == ED_TAPE_ALL ? 7 : std::max(4, 2 * c + 6);
   // CTAs per problem of the streaming kernels: no more than one resident wave over all B
   // problems. Every CTA ends with one to five block sums in FP64 (the narrow pipe here), so at
   // large B fewer, longer CTAs cut that overhead (forward 97 -> 90 ms at B = 64, D = 63,504).
@@ -496,7 +508,7 @@ ed_status bcheck(const ed_plan_s* p, int B, int K, int c) {
   if (p->dim < 1) return fail(ED_ERR_INVALID_ARG, "empty sector");
   if (B < 1 || B > 65535) return fail(ED_ERR_INVALID_ARG, "batch size must be in [1, 65535]");
   if (K < 1 || K > 4096) return fail(ED_ERR_INVALID_ARG, "max_steps must be in [1, 4096]");
-  if (c < 1 || c > 256) return fail(ED_ERR_INVALID_ARG, "checkpoint spacing must be in [1, 256]");
+  if ((c < 1 || c > 256) && c != ED_TAPE_ALL) return fail(ED_ERR_INVALID_ARG, "checkpoint spacing must be in [1, 256]");
   if (p->n_sites > SW_SITES || (int)p->hop.size() > SW_BONDS)
     return fail(ED_ERR_TOO_LARGE, "batched parameters support up to 16 sites and 32 bonds");
   return ED_OK;
@@ -571,7 +583,8 @@ ED_API ed_status ed_batch_lanczos_tape(ed_plan p, int B, const double* d_theta, 
   ED_CUDA(cudaMemsetAsync(d_alpha, 0, (size_t)B * K * sizeof(double), s));
   ED_CUDA(cudaMemsetAsync(d_beta, 0, (size_t)B * (K + 1) * sizeof(double), s));
   const dim3 gv(L.gx, B);
-  auto qv = [&](int k) -> double* { return V + (int64_t)(k % 3) * B * D; };
+  const bool whole = c == ED_TAPE_ALL;
+  auto qv = [&](int k) -> double* { return whole ? d_ckpt + (int64_t)k * B * D : V + (int64_t)(k % 3) * B * D; };
   double* w = V + (int64_t)3 * B * D;
   k_bt_dot<<<gv, BT_NT, 0, s>>>(d_start, d_start, D, part, bs.ticket, n2, 1, d_beta, K + 1, nullptr, 0, 0);
   ED_CHECK_LAUNCH("k_bt_dot");
@@ -602,14 +615,17 @@ ED_API ed_status ed_batch_lanczos_tape(ed_plan p, int B, const double* d_theta, 
     double* q = qv(k);
     double* qp = k > 0 ? qv(k - 1) : nullptr;
     int nl = 4;
-    if (k % c == 0) {
+    if (!whole && k % c == 0) {
       k_bt_ckpt<<<gv, BT_NT, 0, s>>>(q, qp, d_ckpt + (int64_t)(k / c) * 2 * B * D, D, bs.stop);
       ++nl;
     }
     launch_bmv(p, B, d_theta, d_diag, q, w, bs.stop, 1, k, s);
     k_bt_dot<<<gv, BT_NT, 0, s>>>(q, w, D, part, bs.ticket, d_alpha + k, K, nullptr, 0, bs.stop, 1, k);
     k_bt_update<<<gv, BT_NT, 0, s>>>(w, q, qp, D, d_alpha, d_beta, K, k, breakdown, part, bs);
-    k_bt_scale<<<gv, BT_NT, 0, s>>>(w, qv(k + 1), D, d_beta + k + 1, K + 1, bs.stop, 1, k);
+    if (!whole || k + 1 < Km)
+      k_bt_scale<<<gv, BT_NT, 0, s>>>(w, qv(k + 1), D, d_beta + k + 1, K + 1, bs.stop, 1, k);
+    else
+      --nl;
     ED_CHECK_LAUNCH_N("ed_batch_lanczos_tape step", nl);
     if (checks && (k + 1) % check_every == 0 && k + 1 < Km) {
       const int kd = k + 1;
@@ -662,6 +678,12 @@ ED_API ed_status ed_batch_tape_combine(ed_plan p, int B, const double* d_theta, 
   ED_CUDA(cudaMemcpyAsync(bs.m, h_m, B * sizeof(int), cudaMemcpyHostToDevice, s));
   if (d_out) ED_CUDA(cudaMemsetAsync(d_out, 0, (size_t)B * D * sizeof(double), s));
   const dim3 gv(L.gx, B);
+  if (c == ED_TAPE_ALL) {
+    for (int k = 0; k < mmax; ++k)
+      k_bt_acc<<<gv, BT_NT, 0, s>>>(d_ckpt + (int64_t)k * B * D, D, K, k, d_coef, d_out, d_probe, part, bs, d_dots);
+    ED_CHECK_LAUNCH_N("k_bt_acc", mmax);
+    return ED_OK;
+  }
   double* w = V + (int64_t)3 * B * D;
   for (int s0 = 0; s0 < mmax; s0 += c) {
     const int s1 = std::min(s0 + c, mmax);
@@ -715,9 +737,10 @@ ED_API ed_status ed_batch_tape_reverse(ed_plan p, int B, const double* d_theta, 
   double* res = BB + (size_t)B * (K + 1);      // [B]
   const BState bs = bstate(L, base, B);
   const int64_t BD = (int64_t)B * D;
-  double* Qs = V;                   // [c][B][D]
-  double* Ws = V + (int64_t)c * BD; // [c][B][D]
-  double* QB = V + (int64_t)2 * c * BD;
+  const bool whole = c == ED_TAPE_ALL;
+  double* Qs = V;                                       // [c][B][D] (none with a whole tape)
+  double* Ws = whole ? V : V + (int64_t)c * BD;         // [c][B][D] (one)
+  double* QB = whole ? V + BD : V + (int64_t)2 * c * BD;
   double* wbar = QB + 3 * BD;
   double* tmp = wbar + BD;
   double* pracc = tmp + BD;  // [B][D]: sum_k w_bar_k q_k
@@ -734,7 +757,22 @@ ED_API ed_status ed_batch_tape_reverse(ed_plan p, int B, const double* d_theta, 
   ED_CUDA(cudaMemsetAsync(qb(0), 0, BD * sizeof(double), s));
   const SandwichArgs g = sandwich_args(p);
   const dim3 gv(L.gx, B), gw(L.nsw, B);
-  if (mmax > 0) {
+  if (whole) {
+    auto q = [&](int k) -> const double* { return d_ckpt + (int64_t)k * BD; };
+    std::vector<char> ends(mmax + 1, 0);  // the tapes that end after so many steps
+    for (int b = 0; b < B; ++b) ends[h_m[b]] = 1;
+    for (int k = mmax - 1; k >= 0; --k) {
+      const double *q1 = q(k + 1 < mmax ? k + 1 : k), *qm = k > 0 ? q(k - 1) : nullptr;
+      if (ends[k + 1]) launch_bmv(p, B, d_theta, d_diag, q(k), Ws, bs.m, 3, k + 1, s);
+      k_bt_radot<<<gv, BT_NT, 0, s>>>(qb(k + 1), tmp, d_ext_vec, d_ext_coef, q1, q(k), qm, D, d_beta, AB, BB, K, k,
+                                      part, bs, nullptr);
+      k_bt_rstep<<<gw, SW_NT, sandwich_smem(P - 2 * p->n_sites), s>>>(
+          g, p->n_sites, P, qb(k + 1), q1, q(k), qm, Ws, qb(k), k > 0 ? qb(k - 1) : nullptr, wbar, d_alpha, d_beta, AB,
+          BB, K, k, 1, bs, pracc, psw);
+      launch_bmv(p, B, d_theta, d_diag, wbar, tmp, bs.m, 2, k, s);
+      ED_CHECK_LAUNCH_N("ed_batch_tape_reverse step", 3 + ends[k + 1]);
+    }
+  } else if (mmax > 0) {
     const int last_seg = ((mmax - 1) / c) * c;
     for (int s0 = last_seg; s0 >= 0; s0 -= c) {
       const int s1 = std::min(s0 + c, mmax);
@@ -759,16 +797,16 @@ ED_API ed_status ed_batch_tape_reverse(ed_plan p, int B, const double* d_theta, 
         const double* q1 = q(k + 1) ? q(k + 1) : q(k);
         k_bt_radot<<<gv, BT_NT, 0, s>>>(qb(k + 1), tmp, d_ext_vec, d_ext_coef, q1, q(k), k > 0 ? q(k - 1) : nullptr,
                                         D, d_beta, AB, BB, K, k, part, bs, nullptr);
-        k_bt_rstep<<<gw, SW_NT, sandwich_smem(P - 2 * p->n_sites), s>>>(g, p->n_sites, P, qb(k + 1), q1, q(k),
+        k_bt_rstep<<<gw, SW_NT, sandwich_smem(P - 2 * p->n_sites), s>>>(g, p->n_sites, P, qb(k + 1), q1, q(k), nullptr,
                                                       Ws + (int64_t)(k - s0) * BD, qb(k), k > 0 ? qb(k - 1) : nullptr,
-                                                      wbar, d_alpha, d_beta, AB, BB, K, k, bs, pracc, psw);
+                                                      wbar, d_alpha, d_beta, AB, BB, K, k, 0, bs, pracc, psw);
         launch_bmv(p, B, d_theta, d_diag, wbar, tmp, bs.m, 2, k, s);
         ED_CHECK_LAUNCH_N("ed_batch_tape_reverse step", 3);
       }
     }
   }
   // q_bar_0 complete (problems with m >= 1), then the start vectors' adjoints
-  const double* q0 = d_ckpt + BD;
+  const double* q0 = whole ? d_ckpt : d_ckpt + BD;
   k_bt_radot<<<gv, BT_NT, 0, s>>>(qb(0), tmp, d_ext_vec, d_ext_coef, q0, nullptr, nullptr, D, d_beta, AB, BB, K, -1,
                                   part, bs, res);
   k_bt_startbar<<<gv, BT_NT, 0, s>>>(qb(0), q0, D, d_beta, BB, K, res, bs, d_start_bar);

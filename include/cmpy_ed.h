@@ -437,6 +437,8 @@ ED_API ed_status ed_batch_diag(ed_plan plan, int B, const double* d_theta, doubl
 ED_API ed_status ed_batch_matvec_params(ed_plan plan, int B, const double* d_theta,
                                         const double* d_diag, const double* d_x, double* d_y,
                                         ed_stream_t stream);
+/* ckpt = ED_TAPE_ALL: the whole tape, d_ckpt holds q_k at k*B*D for k < max_steps (no replay). */
+#define ED_TAPE_ALL (1 << 30)
 ED_API ed_status ed_batch_tape_workspace(ed_plan plan, int B, int max_steps, int ckpt,
                                          size_t* bytes);
 ED_API ed_status ed_batch_lanczos_tape(ed_plan plan, int B, const double* d_theta,
