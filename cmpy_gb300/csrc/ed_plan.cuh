@@ -66,6 +66,19 @@ struct SpinTable {
   int32_t max_row = 0;        // longest row
 };
 
+// The dn hops in the layout of the FP64 matvec (k_hub_rows_f64): columns in order of their number of hops,
+// and entry e of ordered column j at words[e * n + j] = partner | bond << 16 | (sign < 0) << 31
+struct RowTables {
+  uint32_t* words = nullptr;  // (null: the sector has none)
+  uint16_t* perm = nullptr;   // [n] column of ordered column j
+  uint16_t* cnt = nullptr;    // [n] its hops
+  double* hop = nullptr;      // [bonds]
+  int bonds = 0;
+  int one_hop = 0;            // every hop is t
+  double t = 0.0;
+  int flat = 0;               // every state of a species has the same site energy, and U is uniform
+};
+
 struct FermionParams {
   int n_sites;
   int u_uniform;   // 1 if all u[i] equal (then U-term = u0 * popcount)
@@ -211,6 +224,7 @@ struct ed_plan_s {
   // device tables
   ed::SpinTable up, dn;       // fermion: up/dn species; spin: `up` holds the states
   ed::FermionParams fp;
+  ed::RowTables rows;
   double* spin_diag = nullptr;  // spin: [D]
   ed::DeviceContext* ctx = nullptr;
   ed::BfpTables bfp;
