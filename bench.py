@@ -958,7 +958,7 @@ def run_f64_matvec(steps: int = 20):
     E.lanczos(plan, max_steps=3, want_vector=False)
     r = E.lanczos(plan, max_steps=steps, want_vector=False, profile=True)
     us = 1e3 * r.matvec_ms / max(r.matvecs, 1)
-    return {"workload": "hubbard_ring14_sector77_t0.7_fp64", "kernel": "k_hub_matvec_f64", "matvec_us": round(us, 2),
+    return {"workload": "hubbard_ring14_sector77_t0.7_fp64", "kernel": "k_hub_rows_f64", "matvec_us": round(us, 2),
             "gbs": round(16.0 * plan.dim / (us * 1e-6) / 1e9, 1)}
 
 
