@@ -4,7 +4,8 @@
 //   p_l = (z - a_l) p_{l+1} - b_{l+1}^2 p_{l+2},  value p_1 / p_0,
 // seven FP64 operations a level and no division, where t_l = z - a_l - b_{l+1}^2 / t_{l+1} takes
 // some fifteen. The pipe of this GPU (64 cycles a warp instruction alone, 19 for each when it is full)
-// bounds both. p stays in range by exact powers of two, tested on the exponent bits.
+// bounds both. p is brought back to size one by its own exponent, an exact power of two, whenever it leaves
+// 2^-320 .. 2^320: whatever one level grows by, the next starts in range.
 #pragma once
 
 #include "ed_common.cuh"
@@ -35,9 +36,9 @@ __device__ __forceinline__ double2 cf_value(const double* __restrict__ a, const 
       qi = pi;
       pr = nr;
       pi = ni;
-      const unsigned e = max((unsigned)__double2hiint(pr) & 0x7ff00000u, (unsigned)__double2hiint(pi) & 0x7ff00000u);
-      if (e - 0x2bf00000u > 0x28000000u && e != 0) {  // outside 2^-320 .. 2^320
-        const double sc = e > 0x3ff00000u ? 0x1.0p-320 : 0x1.0p320;
+      const int e = max(__double2hiint(pr) & 0x7ff00000, __double2hiint(pi) & 0x7ff00000);
+      if ((unsigned)(e - 0x2bf00000) > 0x28000000u && e != 0) {  // outside 2^-320 .. 2^320
+        const double sc = __hiloint2double(max(0x7fe00000 - e, 0x00100000), 0);  // 2^-e
         pr *= sc;
         pi *= sc;
         qr *= sc;
