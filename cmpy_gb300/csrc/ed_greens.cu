@@ -145,13 +145,15 @@ __device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
   const double d = b.x * b.x + b.y * b.y;
   return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
 }
-// phi2(x) = (e^x - 1 - x)/x^2 of a complex x; Taylor series for |x| < 1/4. (phi1 = (e^x - 1)/x is
-// 1 + x phi2.) Series: sum x^k/(k+2)!, k < 13: the first term left out is below 0.25^13/15! < 2e-20.
+// phi2(x) = (e^x - 1 - x)/x^2 and phi1 - phi2, phi1(x) = (e^x - 1)/x, of a complex x. |x| < 1/4: the Taylor series
+// of phi2, sum x^k/(k+2)!, k < 13 (the first term left out is below 0.25^13/15! < 2e-20), and phi1 = 1 + x phi2,
+// added in the order (1 - phi2) + x phi2. Elsewhere phi1 by its own quotient: 1 + x phi2 would keep the absolute
+// rounding of 1 in a value of size 1/|x| (a relative error of 2^-53 |x|).
 __constant__ double PHI2_C[13] = {1.0 / 2,         1.0 / 6,          1.0 / 24,          1.0 / 120,
                                   1.0 / 720,       1.0 / 5040,       1.0 / 40320,       1.0 / 362880,
                                   1.0 / 3628800,   1.0 / 39916800,   1.0 / 479001600,   1.0 / 6227020800.0,
                                   1.0 / 87178291200.0};
-__device__ __forceinline__ double2 phi2(double2 x) {
+__device__ __forceinline__ void segment_weights(double2 x, double2* p2, double2* p12) {
   if (x.x * x.x + x.y * x.y < 0.0625) {
     double2 a = make_double2(PHI2_C[12], 0.0);
 #pragma unroll
@@ -159,10 +161,16 @@ __device__ __forceinline__ double2 phi2(double2 x) {
       a = cmul(a, x);
       a.x += PHI2_C[k];
     }
-    return a;
+    const double2 xa = cmul(x, a);
+    *p2 = a;
+    *p12 = make_double2((1.0 - a.x) + xa.x, xa.y - a.y);
+    return;
   }
   const double2 ex = cexp_(x);
-  return cdiv(make_double2(ex.x - 1.0 - x.x, ex.y - x.y), cmul(x, x));
+  const double2 em1 = make_double2(ex.x - 1.0, ex.y);
+  const double2 p1 = cdiv(em1, x);
+  *p2 = cdiv(make_double2(em1.x - x.x, em1.y - x.y), cmul(x, x));
+  *p12 = make_double2(p1.x - p2->x, p1.y - p2->y);
 }
 
 // Laplace transform G(z) = int_{t_0}^{t_{N-1}} e^{i z t} g(t) dt of samples g(t_j), the segments of
@@ -187,10 +195,10 @@ __global__ void __launch_bounds__(LEH_NT) k_laplace_t2z(const double* __restrict
     const double2 ej = cexp_(make_double2(u.x * t[j], u.y * t[j]));
     if (method == 0) {
       const double2 x = make_double2(u.x * h, u.y * h);
-      const double2 p2 = phi2(x);
-      const double2 xp = cmul(x, p2);
+      double2 p2, p12;
+      segment_weights(x, &p2, &p12);
       const double2 c0 = cmul(g[j], p2);
-      const double2 c1 = cmul(g[j + 1], make_double2(1.0 + xp.x - p2.x, xp.y - p2.y));
+      const double2 c1 = cmul(g[j + 1], p12);
       const double2 seg = cmul(ej, make_double2(h * (c0.x + c1.x), h * (c0.y + c1.y)));
       acc.x += seg.x;
       acc.y += seg.y;
