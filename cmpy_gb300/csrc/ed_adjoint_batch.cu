@@ -73,11 +73,10 @@ __device__ __forceinline__ double bhop(double sign, double t) {
   return __longlong_as_double(__double_as_longlong(t) ^ (__double_as_longlong(sign) & (long long)0x8000000000000000ull));
 }
 
-// problem b is skipped when mode 1: gate[b] != 0, mode 2: k >= gate[b], mode 3: k != gate[b]
+// problem b is skipped when mode 1: gate[b] != 0, mode 2: k >= gate[b]
 __device__ __forceinline__ bool bskip(const int* gate, int mode, int k, int b) {
   if (mode == 1) return gate[b] != 0;
   if (mode == 2) return k >= gate[b];
-  if (mode == 3) return k != gate[b];
   return false;
 }
 // the same for all threads of a block (mode 1 gates are set by convergence tests on another stream)
@@ -356,19 +355,16 @@ __global__ void __launch_bounds__(BT_NT) k_bt_radot(double* __restrict__ qb1, co
 
 // reverse step k, part 2, per problem with k < m[b] (the single tape's k_tp_rstep), fused with
 // w_bar^T (dH_b/dtheta) q_k added to the block's row of psw[b][blk][SW_P]
-// whole: every q is on the tape, and w_k = H q_k of a step with a successor is what the recurrence made it,
-// beta_{k+1} q_{k+1} + alpha_k q_k + beta_k q_{k-1}: three FP64 operations an element, H takes eleven.
 // (Bound by the FP64 pipe. The accumulators are those of the hop parameters alone: with the 2 ns rows
 // that stay zero here, zeroing and adding them up was a third of the kernel's FP64 instructions and its shared
 // memory kept half of the warps off an SM. With tp_block_rows in k_bt_radot, 64 problems of 63,504
 // states, forward and backward: 308 -> 269 ms.)
 __global__ void __launch_bounds__(SW_NT) k_bt_rstep(SandwichArgs g, int ns, int P, const double* __restrict__ qb1,
                                                     const double* __restrict__ q1, const double* __restrict__ q0,
-                                                    const double* __restrict__ qm, const double* __restrict__ w0,
-                                                    double* __restrict__ qbk, double* __restrict__ qbm,
-                                                    double* __restrict__ wbar, const double* alpha,
-                                                    const double* beta, const double* abar, const double* bbar, int K,
-                                                    int k, int whole, BState bs,
+                                                    const double* __restrict__ w0, double* __restrict__ qbk,
+                                                    double* __restrict__ qbm, double* __restrict__ wbar,
+                                                    const double* alpha, const double* beta, const double* abar,
+                                                    const double* bbar, int K, int k, BState bs,
                                                     double* __restrict__ pracc, double* __restrict__ psw) {
   const int b = blockIdx.y;
   const int m = bs.m[b];
@@ -378,8 +374,7 @@ __global__ void __launch_bounds__(SW_NT) k_bt_rstep(SandwichArgs g, int ns, int 
   sandwich_zero(sacc, nb);
   const bool has_next = k + 1 < m, first = k == m - 1;
   const double ak = alpha[(int64_t)b * K + k], ab = abar[(int64_t)b * K + k];
-  const double b1 = has_next ? beta[(int64_t)b * (K + 1) + k + 1] : 0.0;
-  const double inv = has_next ? 1.0 / b1 : 0.0;
+  const double inv = has_next ? 1.0 / beta[(int64_t)b * (K + 1) + k + 1] : 0.0;
   const double bb1 = has_next ? bbar[(int64_t)b * (K + 1) + k + 1] : 0.0;
   const double bk = k > 0 ? beta[(int64_t)b * (K + 1) + k] : 0.0;
   const int64_t D = g.nu * g.nd, o = (int64_t)b * D;
@@ -388,14 +383,7 @@ __global__ void __launch_bounds__(SW_NT) k_bt_rstep(SandwichArgs g, int ns, int 
     const double rb = has_next ? fma(bb1, q1[o + i], qb1[o + i] * inv) : 0.0;
     const double x0 = q0b[i];
     const double wb = fma(ab, x0, rb);
-    double w;
-    if (whole && has_next) {
-      w = fma(b1, q1[o + i], ak * x0);
-      if (qm) w = fma(bk, qm[o + i], w);
-    } else {
-      w = w0[o + i];
-    }
-    qbk[o + i] = fma(ab, w, fma(-ak, rb, first ? 0.0 : qbk[o + i]));
+    qbk[o + i] = fma(ab, w0[o + i], fma(-ak, rb, first ? 0.0 : qbk[o + i]));
     if (qbm) qbm[o + i] = -bk * rb;
     wbar[o + i] = wb;
     // the hop part now, the diagonal part through sum_k w_bar_k q_k
@@ -758,19 +746,18 @@ ED_API ed_status ed_batch_tape_reverse(ed_plan p, int B, const double* d_theta, 
   const SandwichArgs g = sandwich_args(p);
   const dim3 gv(L.gx, B), gw(L.nsw, B);
   if (whole) {
+    // (w_k = H q_k is applied as in the replays, so that either tape gives the same bits)
     auto q = [&](int k) -> const double* { return d_ckpt + (int64_t)k * BD; };
-    std::vector<char> ends(mmax + 1, 0);  // the tapes that end after so many steps
-    for (int b = 0; b < B; ++b) ends[h_m[b]] = 1;
     for (int k = mmax - 1; k >= 0; --k) {
       const double *q1 = q(k + 1 < mmax ? k + 1 : k), *qm = k > 0 ? q(k - 1) : nullptr;
-      if (ends[k + 1]) launch_bmv(p, B, d_theta, d_diag, q(k), Ws, bs.m, 3, k + 1, s);
+      launch_bmv(p, B, d_theta, d_diag, q(k), Ws, bs.m, 2, k, s);
       k_bt_radot<<<gv, BT_NT, 0, s>>>(qb(k + 1), tmp, d_ext_vec, d_ext_coef, q1, q(k), qm, D, d_beta, AB, BB, K, k,
                                       part, bs, nullptr);
       k_bt_rstep<<<gw, SW_NT, sandwich_smem(P - 2 * p->n_sites), s>>>(
-          g, p->n_sites, P, qb(k + 1), q1, q(k), qm, Ws, qb(k), k > 0 ? qb(k - 1) : nullptr, wbar, d_alpha, d_beta, AB,
-          BB, K, k, 1, bs, pracc, psw);
+          g, p->n_sites, P, qb(k + 1), q1, q(k), Ws, qb(k), k > 0 ? qb(k - 1) : nullptr, wbar, d_alpha, d_beta, AB, BB,
+          K, k, bs, pracc, psw);
       launch_bmv(p, B, d_theta, d_diag, wbar, tmp, bs.m, 2, k, s);
-      ED_CHECK_LAUNCH_N("ed_batch_tape_reverse step", 3 + ends[k + 1]);
+      ED_CHECK_LAUNCH_N("ed_batch_tape_reverse step", 4);
     }
   } else if (mmax > 0) {
     const int last_seg = ((mmax - 1) / c) * c;
@@ -797,9 +784,9 @@ ED_API ed_status ed_batch_tape_reverse(ed_plan p, int B, const double* d_theta, 
         const double* q1 = q(k + 1) ? q(k + 1) : q(k);
         k_bt_radot<<<gv, BT_NT, 0, s>>>(qb(k + 1), tmp, d_ext_vec, d_ext_coef, q1, q(k), k > 0 ? q(k - 1) : nullptr,
                                         D, d_beta, AB, BB, K, k, part, bs, nullptr);
-        k_bt_rstep<<<gw, SW_NT, sandwich_smem(P - 2 * p->n_sites), s>>>(g, p->n_sites, P, qb(k + 1), q1, q(k), nullptr,
+        k_bt_rstep<<<gw, SW_NT, sandwich_smem(P - 2 * p->n_sites), s>>>(g, p->n_sites, P, qb(k + 1), q1, q(k),
                                                       Ws + (int64_t)(k - s0) * BD, qb(k), k > 0 ? qb(k - 1) : nullptr,
-                                                      wbar, d_alpha, d_beta, AB, BB, K, k, 0, bs, pracc, psw);
+                                                      wbar, d_alpha, d_beta, AB, BB, K, k, bs, pracc, psw);
         launch_bmv(p, B, d_theta, d_diag, wbar, tmp, bs.m, 2, k, s);
         ED_CHECK_LAUNCH_N("ed_batch_tape_reverse step", 3);
       }
