@@ -121,8 +121,7 @@ def case_adjoint64(n: int = 64) -> None:
     rows = [siam_parameters(u, e_imp, eb[i], v[i]) for i in range(n)]
     th = torch.stack([r[0] for r in rows])
     n_sites, bonds, width = rows[0][1], rows[0][2], rows[0][3]
-    g = greens_function_ad_batch(th, n_sites, bonds, (5, 5), z, sign_width=width, gs_steps=250, gf_levels=150,
-                                 ckpt=16)
+    g = greens_function_ad_batch(th, n_sites, bonds, (5, 5), z, sign_width=width, gs_steps=250, gf_levels=150)
     torch.sum(torch.abs(g) ** 2).backward()
     torch.cuda.synchronize()
     print(f"adjoint64: |grad| = {float(eb.grad.abs().sum() + v.grad.abs().sum()):.6f}")
@@ -587,7 +586,7 @@ def run_adjoint(n_siam: int = 64, n_freq: int = 1024, n_single: int = 8):
     v = torch.tensor(rng.uniform(0.1, 0.6, (n_siam, 9)), dtype=torch.float64, device="cuda", requires_grad=True)
     u = torch.tensor(4.0, dtype=torch.float64, device="cuda")
     e_imp = torch.tensor(0.0, dtype=torch.float64, device="cuda")
-    kw = dict(gs_steps=250, gf_levels=150, ckpt=16)
+    kw = dict(gs_steps=250, gf_levels=150)
 
     def thetas():
         rows = [siam_parameters(u, e_imp, eb[i], v[i]) for i in range(n_siam)]

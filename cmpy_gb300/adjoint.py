@@ -294,24 +294,38 @@ def batch_matvec(plan: E.Plan, thetas: torch.Tensor, diag: torch.Tensor, x: torc
 TAPE_ALL = 1 << 30  # (ED_TAPE_ALL: no checkpoints, the whole tape)
 
 
+class _DefaultSpacing(int):
+    """The checkpoint spacing of a call that names none, told by its type from a caller's own number."""
+
+
+CKPT = _DefaultSpacing(16)
+
+
+def _check_spacing(c: int) -> int:
+    if not 1 <= c <= 256:
+        raise ValueError("checkpoint spacing must be in [1, 256]")
+    return c
+
+
 def _tape_spacing(c: int, vector_bytes: int, K: int) -> int:
     """c, or TAPE_ALL where all Krylov vectors together take at most a sixteenth of the memory that an allocation
     can have (the driver's free memory and what PyTorch holds without use): without the replays and the matvecs
     that they take (64 problems of 63,504 states, three tapes of 16 GB together: 269 -> 234 ms). A sixteenth,
     because the three tapes of a call stay until its backward and other calls' may lie beside them: each leaves
     the next fifteen sixteenths of what it found. Either tape gives the same bits."""
-    if not 1 <= c <= 256:
-        raise ValueError("checkpoint spacing must be in [1, 256]")
+    _check_spacing(c)
     free = torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
     return TAPE_ALL if K * vector_bytes <= free // 16 else c
 
 
 def batch_tape_forward(plan: E.Plan, thetas: torch.Tensor, diag: torch.Tensor, starts: torch.Tensor, max_steps: int,
-                       c: int = 16, tol: float = 0.0, check_every: int = 10,
-                       breakdown: float = 1e-13) -> BatchTape:
+                       c: int = CKPT, tol: float = 0.0, check_every: int = 10,
+                       breakdown: float = 1e-13, whole: bool = True) -> BatchTape:
+    """Tapes of B Lanczos runs; whole: every Krylov vector instead of checkpoints c steps apart where memory
+    allows."""
     B = thetas.shape[0]
     K = int(min(max_steps, plan.dim))
-    c = _tape_spacing(int(c), 8 * B * plan.dim, K)
+    c = _tape_spacing(int(c), 8 * B * plan.dim, K) if whole else _check_spacing(int(c))
     nb = C.c_size_t()
     N.check(N.lib().ed_batch_tape_workspace(plan.handle, B, K, c, C.byref(nb)))
     work = torch.empty(int(nb.value), dtype=torch.uint8, device=E.device())
@@ -402,8 +416,10 @@ def _apply_fermion_rows(src: E.Plan, dst: E.Plan, pos: int, sigma: int, create: 
     return Y
 
 
-def _gf_forward_batch(thetas: torch.Tensor, spec, zt: torch.Tensor, g: torch.Tensor):
-    n_sites, bonds, width, (nu, nd), pos, sigma, m0, mgf, c, seed = spec
+def _gf_forward_batch(thetas: torch.Tensor, spec, zt: torch.Tensor, g: torch.Tensor, grad: bool):
+    """grad: a backward may follow (the neighbours' vectors are read by it alone)."""
+    n_sites, bonds, width, (nu, nd), pos, sigma, m0, mgf, ckpt, seed = spec
+    c, whole = int(ckpt), isinstance(ckpt, _DefaultSpacing)
     B = thetas.shape[0]
     th = thetas.detach().to(dtype=torch.float64).contiguous()
     dev = E.device()
@@ -411,7 +427,7 @@ def _gf_forward_batch(thetas: torch.Tensor, spec, zt: torch.Tensor, g: torch.Ten
     diag = batch_diag(plan, th)
     gen = torch.Generator(device="cpu").manual_seed(seed)
     v0 = torch.rand(plan.dim, generator=gen, dtype=torch.float64).to(dev)
-    tape0 = batch_tape_forward(plan, th, diag, v0.expand(B, -1), m0, c, tol=1e-12)
+    tape0 = batch_tape_forward(plan, th, diag, v0.expand(B, -1), m0, c, tol=1e-12, whole=whole)
     e0_d, cvec = E.tridiag_lowest_batch(tape0.alpha, tape0.beta, tape0.m)
     e0 = e0_d.cpu().numpy()
     Y, _ = batch_tape_combine(tape0, coef=cvec)
@@ -425,7 +441,7 @@ def _gf_forward_batch(thetas: torch.Tensor, spec, zt: torch.Tensor, g: torch.Ten
             continue
         tp = structure_plan(n_sites, bonds, width, tu, td)
         start = _apply_fermion_rows(plan, tp, pos, sigma, create, psi)
-        tape = batch_tape_forward(tp, th, batch_diag(tp, th), start, mgf, c)
+        tape = batch_tape_forward(tp, th, batch_diag(tp, th), start, mgf, c, whole=whole and grad)
         n2 = tape.beta[:, 0].cpu().numpy() ** 2
         batch_cf(tape, n2, e0, sign, zt, g)
         parts.append((tp, tape, sign, create, n2))
@@ -474,15 +490,15 @@ class GreensFunctionADBatch(torch.autograd.Function):
     problems in one launch per kernel."""
 
     @staticmethod
-    def forward(ctx, thetas, spec, z):
+    def forward(ctx, thetas, spec, z, grad=True):
         zt = E._as_dev_c128(z)
         g = torch.zeros((thetas.shape[0], zt.numel()), dtype=torch.complex128, device=E.device())
-        ctx.saved = _gf_forward_batch(thetas, spec, zt, g)
+        ctx.saved = _gf_forward_batch(thetas, spec, zt, g, grad)
         return g
 
     @staticmethod
     def backward(ctx, gbar):
-        return _gf_backward_batch(ctx.saved, gbar).to(gbar.device), None, None
+        return _gf_backward_batch(ctx.saved, gbar).to(gbar.device), None, None, None
 
 
 def greens_function_ad(theta: torch.Tensor, n_sites: int, bonds, sector, z, pos: int = 0, sigma: int = 1,
@@ -496,17 +512,20 @@ def greens_function_ad(theta: torch.Tensor, n_sites: int, bonds, sector, z, pos:
 
 def greens_function_ad_batch(thetas: torch.Tensor, n_sites: int, bonds, sector, z, pos: int = 0, sigma: int = 1,
                              sign_width: int | None = None, gs_steps: int = 200, gf_levels: int = 200,
-                             ckpt: int = 16, seed: int = 0) -> torch.Tensor:
+                             ckpt: int = CKPT, seed: int = 0) -> torch.Tensor:
     """Differentiable T=0 G(z) of B models with one structure (thetas[B, P], rows as in
     greens_function_ad) -> [B, n_z]. Each problem follows the arithmetic of greens_function_ad;
-    every Lanczos step of all B problems runs as one launch per kernel (batched tape)."""
+    every Lanczos step of all B problems runs as one launch per kernel (batched tape).
+    ckpt: steps between the tape's checkpoints, which bound its memory (2 / ckpt of the Krylov vectors, and
+    2 ckpt + 6 vectors of workspace); a call that names none keeps 16 or, where they take at most a sixteenth of
+    the memory that is left, every vector. G and its gradient have the same bits with every choice."""
     spec = (n_sites, [tuple(b) for b in bonds], n_sites if sign_width is None else sign_width, tuple(sector), pos,
             sigma, gs_steps, gf_levels, ckpt, seed)
     if thetas.dim() != 2:
         raise ValueError("thetas must be [B, P]")
     if thetas.shape[1] != 2 * n_sites + len(spec[1]):
         raise ValueError("thetas must have 2 * n_sites + n_bonds columns")
-    return GreensFunctionADBatch.apply(thetas, spec, z)
+    return GreensFunctionADBatch.apply(thetas, spec, z, torch.is_grad_enabled() and thetas.requires_grad)
 
 
 def siam_parameters(u, eps_imp, eps_bath, v, mu=None):
