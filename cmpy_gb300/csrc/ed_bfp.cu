@@ -1739,8 +1739,7 @@ static int matvec_variant(const ed_plan_s* p) {
 // when the environment asks for it
 ed_status build_default_two_pass(ed_plan_s* p, cudaStream_t s) {
   if (!p->bfp.eligible) return ED_OK;
-  const char* e = getenv("CMPY_ED_MATVEC");
-  const int forced = e ? atoi(e) : 0;
+  const int forced = forced_variant(p);  // (the environment's: read once per process)
   return build_two_pass(p, forced == 5 || matvec_variant(p) < 3, forced == 6, s);
 }
 
