@@ -156,6 +156,7 @@ _SIGNATURES = {
         [C.c_void_p, I32, F64, I32, C.c_uint64, P, I32, P, C.c_size_t, P, P, P, P, P, P, P, I32, I32, I32, P],
     ),
     "ed_batch_lanczos_coeffs": (I32, [C.c_void_p, I32, C.c_uint64, P, P, C.c_size_t, P, P, P, I32, I32, I32, P]),
+    "ed_batch_resident": (I32, [C.c_void_p, I32, I32, I32]),
     "ed_batch_tune": (
         I32,
         [C.c_void_p, I32, P, C.c_size_t, P, P, P, P, P, C.POINTER(I32), C.POINTER(I32), C.POINTER(I32),

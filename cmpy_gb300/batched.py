@@ -108,6 +108,10 @@ class Batch:
         _tune_cache[key] = (self.threads, self.ctas_per_sm, self.cluster_size, float(ms.value))
         return _tune_cache[key]
 
+    def resident(self, threads: int, ctas_per_sm: int, cluster_size: int) -> bool:
+        """Whether the launch configuration keeps every problem's vectors in shared memory."""
+        return bool(N.lib().ed_batch_resident(self._h, int(threads), int(ctas_per_sm), int(cluster_size)))
+
     def _starts(self, starts):
         """Device array of the start vectors' pointers (None: seeded starts)."""
         if starts is None:

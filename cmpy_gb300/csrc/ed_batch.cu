@@ -3,8 +3,6 @@
 #include "ed_batch.cuh"
 #include "ed_cf.cuh"
 
-#include "ed_resident.cuh"
-
 namespace ed {
 
 // G_p(z) += sign * norm_p^2 / (z' - a0 - b1^2 / (z' - a1 - ...)),  z' = sign*z + e0_p,
@@ -68,6 +66,12 @@ static bool valid_config(int threads, int per_sm, int cs) {
   return t_ok && c_ok && per_sm >= 1 && per_sm <= 16;
 }
 
+// threads of the kernel that a request for `threads` takes: with one CTA per problem whole columns of the sums
+// (RES_COLS) and a warp for the scalars
+static int kernel_threads(int threads, int cs) {
+  return cs > 1 ? threads : (threads <= 256 ? 288 : (threads == 512 ? 544 : 800));
+}
+
 static ed_status run_batch(const ed_batch_s* b, int threads, int per_sm, int cs, int K, double tol, int check_every,
                            uint64_t seed, const double* const* starts, int want_vector, void* work, size_t bytes,
                            const BatchOut& out, cudaStream_t s) {
@@ -87,10 +91,10 @@ static ed_status run_batch(const ed_batch_s* b, int threads, int per_sm, int cs,
   ED_CUDA(cudaMemsetAsync(wk.queue, 0, sizeof(int), s));
 #define ED_BATCH_CASE(NT, CS) \
   if (threads == NT && cs == CS) return launch_batch<NT, CS>(b, grid, per_sm, K, tol, check_every, seed, starts, want_vector, out, wk, s);
-  // one CTA per problem: whole columns of the sums (RES_COLS) and a warp for the scalars
   if (cs == 1) {
-    if (threads <= 256) return launch_batch<288, 1>(b, grid, per_sm, K, tol, check_every, seed, starts, want_vector, out, wk, s);
-    if (threads == 512) return launch_batch<544, 1>(b, grid, per_sm, K, tol, check_every, seed, starts, want_vector, out, wk, s);
+    const int nt = kernel_threads(threads, 1);
+    if (nt == 288) return launch_batch<288, 1>(b, grid, per_sm, K, tol, check_every, seed, starts, want_vector, out, wk, s);
+    if (nt == 544) return launch_batch<544, 1>(b, grid, per_sm, K, tol, check_every, seed, starts, want_vector, out, wk, s);
     return launch_batch<800, 1>(b, grid, per_sm, K, tol, check_every, seed, starts, want_vector, out, wk, s);
   }
   ED_BATCH_CASE(512, 2)
@@ -183,6 +187,15 @@ ED_API ed_status ed_batch_destroy(ed_batch b) {
   cudaFree(b->d_order);
   delete b;
   return ED_OK;
+}
+
+ED_API int ed_batch_resident(ed_batch b, int threads, int ctas_per_sm, int cluster_size) {
+  if (!b || !valid_config(threads, ctas_per_sm, cluster_size)) return 0;
+  const int nt = kernel_threads(threads, cluster_size);
+  const size_t budget = batch_smem(b, nt, cluster_size, ctas_per_sm);
+  for (const auto& q : b->shapes)
+    if (!res_layout(q.nu, q.nd, q.quads, nt, cluster_size, budget).ws) return 0;
+  return 1;
 }
 
 ED_API ed_status ed_batch_workspace(ed_batch b, int max_steps, int threads, int ctas_per_sm, int cluster_size,

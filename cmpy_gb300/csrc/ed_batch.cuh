@@ -31,10 +31,9 @@
 #include <vector>
 
 #include "ed_plan.cuh"
+#include "ed_resident.cuh"
 
 namespace ed {
-struct BatchProblem;
-
 struct BatchOut {
   double* alpha;     // [n][K]
   double* beta;      // [n][K+1]; beta[p][0] = start norm, beta[p][k>0] couplings
@@ -80,6 +79,20 @@ template <int NT, int CS>
 ed_status launch_batch(const ed_batch_s* b, int grid, int per_sm, int K, double tol, int check_every, uint64_t seed,
                        const double* const* starts, int want_vector, const BatchOut& out, const BatchWork& wk,
                        cudaStream_t s);
+// Dynamic shared memory of a CTA when per_sm of them share an SM: as much as that leaves, but no more
+// than the batch's largest need (a problem that does not fit keeps R or all its vectors in its
+// global slots).
+constexpr size_t RES_STATIC = 5 * 1024;  // bound of the kernel's static shared memory
+static inline size_t batch_smem(const ed_batch_s* b, int NT, int CS, int per_sm) {
+  const size_t sm = (size_t)b->ctx->smem_optin + 1024;  // one CTA's limit plus the system's share
+  const size_t per = sm / per_sm;
+  if (per <= RES_STATIC + 1024) return 0;
+  const size_t budget = (per - RES_STATIC - 1024) / 1024 * 1024;
+  size_t need = 0;
+  for (const auto& q : b->shapes) need = std::max(need, res_layout(q.nu, q.nd, q.quads, NT, CS, budget).total);
+  return need;
+}
+
 // how many clusters of cs CTAs of the NT-thread kernel the device can hold at once (0: none)
 template <int NT, int CS>
 int clusters_for();

@@ -2,7 +2,6 @@
 #pragma once
 
 #include "ed_batch.cuh"
-#include "ed_resident.cuh"
 
 namespace ed {
 
@@ -63,20 +62,6 @@ __global__ void __launch_bounds__(NT, NT == 288 ? 3 : (NT <= 544 ? 2 : 1)) k_bat
     csync<CS>();  // the cluster's slots and P are free for the next problem
   }
   csync<CS>();  // no CTA leaves while another may still read its shared memory
-}
-
-// Dynamic shared memory of a CTA when per_sm of them share an SM: as much as that leaves, but no more
-// than the batch's largest need (a problem that does not fit keeps R or all its vectors in its
-// global slots).
-constexpr size_t RES_STATIC = 5 * 1024;  // bound of the kernel's static shared memory
-static inline size_t batch_smem(const ed_batch_s* b, int NT, int CS, int per_sm) {
-  const size_t sm = (size_t)b->ctx->smem_optin + 1024;  // one CTA's limit plus the system's share
-  const size_t per = sm / per_sm;
-  if (per <= RES_STATIC + 1024) return 0;
-  const size_t budget = (per - RES_STATIC - 1024) / 1024 * 1024;
-  size_t need = 0;
-  for (const auto& q : b->shapes) need = std::max(need, res_layout(q.nu, q.nd, q.quads, NT, CS, budget).total);
-  return need;
 }
 
 template <int NT, int CS>

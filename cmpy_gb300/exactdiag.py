@@ -86,7 +86,9 @@ def _resident_energies(model, fillings, max_steps: int, tol: float, check_every:
     """{filling: (energy, None)} of the sectors whose Lanczos runs fit a cluster's shared memory, all in
     one launch; the same start vectors as groundstate_sector's. The cluster of a sector is as large as
     keeps every sector's running at once (a single run: 400 states 5.6 us a step on 2 CTAs, 5.8 on 8;
-    4900 states 12.6, 8.2, 7.7 on 2, 4, 8)."""
+    4900 states 12.6, 8.2, 7.7 on 2, 4, 8), or the smallest that still holds the largest sector's vectors:
+    the 80 sectors of the 9-site chain (15,876 states at most, one CTA to an SM) on clusters of 2, whose
+    vectors are in global memory, 6.95 ms, of 4, in two waves, 5.72, of 8 10.64."""
     from .batched import Batch
 
     n = model.num_sites
@@ -97,9 +99,10 @@ def _resident_energies(model, fillings, max_steps: int, tol: float, check_every:
     batch = Batch([p for _, p in pairs])
     dmax = max(batch.dims)
     sms = torch.cuda.get_device_properties(E.device()).multi_processor_count
-    # (two CTAs to an SM while the vectors of the largest sector, 10 bytes a state, leave room for two)
+    # (two CTAs to an SM while the vectors of the largest sector, 10 bytes a state on 8 CTAs, leave room for two)
     batch.threads, batch.ctas_per_sm = 512, 2 if dmax <= 8000 else 1
-    batch.cluster_size = next((c for c in (8, 4) if len(pairs) * c <= sms * batch.ctas_per_sm), 2)
+    fits = [c for c in (8, 4, 2) if batch.resident(512, batch.ctas_per_sm, c)] or [8]
+    batch.cluster_size = next((c for c in fits if len(pairs) * c <= sms * batch.ctas_per_sm), fits[-1])
     x = E.random_start(dmax)
     res = batch.lanczos(min(max_steps, dmax), tol, check_every, starts=[x[:d] for d in batch.dims])
     return {f: (energy, None) for (f, _), energy in zip(pairs, res.energy.tolist())}

@@ -377,6 +377,9 @@ ED_API ed_status ed_batch_tune(ed_batch batch, int tune_steps, void* d_work, siz
                                double* d_residual, int32_t* d_steps, int* h_threads,
                                int* h_ctas_per_sm, int* h_cluster_size, float* h_ms,
                                ed_stream_t stream);
+/* 1 when the launch configuration keeps the tables and vectors of every problem in shared memory (a
+ * cluster's CTA holds R and its share of W and R_{k-1}: 8 + 16 / cluster_size bytes a state), else 0. */
+ED_API int ed_batch_resident(ed_batch batch, int threads, int ctas_per_sm, int cluster_size);
 /* Adds the continued fraction of every problem (layout of ed_batch_lanczos, norm^2 =
  * beta[p*(K+1)]^2, shift d_e0[p]) at n_z frequencies into d_g[p*n_z + j] (complex FP64). */
 ED_API ed_status ed_batch_gf_continued_fraction(int n, int max_steps, const double* d_alpha,
