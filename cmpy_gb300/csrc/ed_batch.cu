@@ -7,7 +7,7 @@ namespace ed {
 
 // G_p(z) += sign * norm_p^2 / (z' - a0 - b1^2 / (z' - a1 - ...)),  z' = sign*z + e0_p,
 // norm_p = beta[p][0] (start norm), m_p = steps[p]; one thread per frequency, one problem per
-// blockIdx.y. Bound by the FP64 pipe: 512 problems x 1280 frequencies x 2000 levels 28.7 -> 22.9 ms.
+// blockIdx.y. Bound by the FP64 pipe: 512 problems x 1280 frequencies x 2000 levels 32.9 -> 26.4 ms.
 constexpr int BCF_NT = 128;
 __global__ void __launch_bounds__(BCF_NT) k_batch_cf(int n, int K, const double* __restrict__ alpha,
                                                      const double* __restrict__ beta, const int32_t* __restrict__ steps,

@@ -14,11 +14,12 @@
 // exponent per vector, exact integer matvec, 128-bit dot products).
 //
 // With a thread-block cluster of CS > 1 CTAs per problem, the cluster's CTAs split the
-// elements of every vector loop (CTA rank r takes the r-th stripe of CS * NT) and exchange their
-// block totals through distributed shared memory at the hardware cluster barrier; every CTA
-// then holds the same totals and computes the same scalars, so all CTAs of a cluster take the
-// same branches and reach the same barriers. The largest sectors, which bound the makespan of
-// the work queue, thus run on CS SMs.
+// elements of every vector loop (CTA rank r takes the r-th stripe of the CS * (NT - 32) that own
+// elements) and exchange their block totals through distributed shared memory at the hardware cluster
+// barrier; every CTA then holds the same totals and computes the same scalars, an invariant subspace
+// among them. The convergence tests are CTA 0's alone: the others wait for it at a cluster barrier and
+// take its stop flag. So all CTAs of a cluster take the same branches and reach the same barriers. The
+// largest sectors, which bound the makespan of the work queue, thus run on CS SMs.
 //
 // This header holds the kernel and its launch; ed_batch_one.cu and ed_batch_c{2,4,8}.cu instantiate them (one
 // translation unit each, compiled in parallel), ed_batch.cu has the entry points.
@@ -47,7 +48,7 @@ struct BatchOut {
 struct BatchWork {
   int64_t* slots;     // per CTA: Ra, Rb, W, acc_lo, acc_hi (each dmax)
   int64_t dmax;
-  double* tri;        // per CTA: 6*(K+2) doubles (tridiagonal work + eigenvector)
+  double* tri;        // per CTA: 8*(K+2) doubles (tridiagonal work 5, eigenvector, alpha, beta)
   int32_t* exps;      // per CTA: K+2 exponents of R_k
   int64_t* coefs;     // per CTA: K+2 Ritz coefficients
   int* queue;

@@ -14,7 +14,7 @@ namespace ed {
 
 // G(z) = sign * norm2 / (z' - a0 - b1^2 / (z' - a1 - ...)),  z' = sign * z + shift; one thread per
 // frequency, blocks of one warp (a few thousand frequencies are spread over the SMs, whose FP64 pipes a
-// single warp each already holds: 200 levels at 2048 frequencies 118 -> 84 us)
+// single warp each already holds: 200 levels at 2048 frequencies 120 -> 87 us)
 constexpr int CF_NT = 32;
 __global__ void __launch_bounds__(CF_NT) k_cf(const double* __restrict__ a, const double* __restrict__ b, int n,
                                               double norm2, double shift, int sign, const double2* __restrict__ z,

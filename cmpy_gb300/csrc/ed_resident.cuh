@@ -17,8 +17,8 @@
 //
 // Sums. One CTA: the elements go to 256 columns (i mod 256) whose exact sums are rounded to FP64 and
 // added in one fixed order, whatever the number of threads, so every configuration gives the same
-// bits. A cluster: the exact total, rounded once (a warp adds the 128-bit values as 26-bit limbs with the
-// integer reduction instruction).
+// bits. A cluster: the exact total (a warp adds the 128-bit values as 26-bit limbs with the integer
+// reduction instruction), converted to FP64 from its high and low words, each rounded, and their sum.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -109,11 +109,6 @@ __device__ __forceinline__ Wide warp_sum_wide(const I128& v) {
 }
 __device__ __forceinline__ Wide warp_sum_wide(const Wide& v) {
   return warp_sum_wide(v.lo, v.hi, v.top + (int)(v.hi >> 40));
-}
-__device__ __forceinline__ void add_wide(Wide& a, const Wide& b) {
-  a.lo += b.lo;
-  a.hi += b.hi + (a.lo < b.lo ? 1u : 0u);
-  a.top += b.top;
 }
 // (the magnitude is converted: no cancellation between the words)
 __device__ __forceinline__ double wide_to_double(const Wide& v) {

@@ -88,7 +88,7 @@ def _resident_energies(model, fillings, max_steps: int, tol: float, check_every:
     keeps every sector's running at once (a single run: 400 states 5.6 us a step on 2 CTAs, 5.8 on 8;
     4900 states 12.6, 8.2, 7.7 on 2, 4, 8), or the smallest that still holds the largest sector's vectors:
     the 80 sectors of the 9-site chain (15,876 states at most, one CTA to an SM) on clusters of 2, whose
-    vectors are in global memory, 6.95 ms, of 4, in two waves, 5.72, of 8 10.64."""
+    vectors are in global memory, 6.95 ms, of 4, not all at once, 5.72, of 8 10.64."""
     from .batched import Batch
 
     n = model.num_sites

@@ -366,10 +366,14 @@ ED_API ed_status ed_batch_lanczos_coeffs(ed_batch b, int max_steps, uint64_t see
                                          int32_t* d_steps, int threads, int ctas_per_sm, int cluster_size,
                                          ed_stream_t stream);
 
-/* Launch configuration: threads per CTA (128, 256, 512, 1024), CTAs per SM, and the
+/* Launch configuration: threads per CTA (128, 256, 512, 1024), CTAs per SM (1 to 16), and the
  * thread-block cluster size per problem (1, or 2/4/8 with 512 or 1024 threads: the cluster's
  * CTAs share each problem's vectors and exchange their partial sums through distributed
- * shared memory). threads <= 0 selects the tuned (or default) configuration.
+ * shared memory). With one CTA per problem the kernels have a warp for the scalars beside whole
+ * columns of the sums: 128 and 256 select the one of 288 threads, 512 of 544, 1024 of 800. CTAs per SM
+ * sizes the grid and each CTA's share of shared memory; the registers let 3, 2 and 1 of these kernels
+ * share an SM (2 and 1 of the cluster kernels of 512 and 1024), more wait their turn.
+ * threads <= 0 selects the tuned (or default) configuration.
  * Autotuner: times the candidate configurations on a tune_steps run and keeps the fastest for
  * this batch (used when ed_batch_lanczos gets threads <= 0). Synchronous. */
 ED_API ed_status ed_batch_tune(ed_batch batch, int tune_steps, void* d_work, size_t work_bytes,
