@@ -200,11 +200,16 @@ class AbstractManyBodyModel(AbstractModel):
         return None
 
     def plan(self, n_up: int, n_dn: int) -> "E.Plan":
-        return self.plans([(n_up, n_dn)])[0]
+        return self._sector_plans([(n_up, n_dn)])[0]
 
     def plans(self, sectors) -> list:
         """Plans of several (n_up, n_dn) sectors of the current parameters (one descriptor for
-        all of them); a None entry gives None."""
+        all of them, or each from ``plan`` where a subclass defines its own); a None entry gives None."""
+        if type(self).plan is not AbstractManyBodyModel.plan:
+            return [None if sec is None else self.plan(int(sec[0]), int(sec[1])) for sec in sectors]
+        return self._sector_plans(sectors)
+
+    def _sector_plans(self, sectors) -> list:
         desc = self.fermion_descriptor()
         if desc is None:
             raise NotImplementedError(f"{type(self).__name__} has no engine descriptor")
